@@ -146,10 +146,18 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
                 const FispLaunch L = tuned_fisp_launch(seq.max_state, V, P);
                 D = L.config < 0 ? fisp_default_launch(seq.max_state, V, P) : L;
             }
-            // jobs with real phases form their own groups, which a packed layout runs in its real-phase form
-            const bool packed = tan ? fisp_tangent_config_packed(D.config) : fisp_config_packed(D.config);
-            const int real = packed && fisp_sequence_real_phases(ctx, seq) ? 1 : 0;
-            keyed.push_back({Key {tan, D.config, std::max(1, std::min(D.warps, 8)), seq.max_state, real}, j});
+            // jobs with real phases form their own groups, on the real-phase kernels (an item of the
+            // queue is up to 4 tiles)
+            const int real = fisp_real_covers(seq) && fisp_sequence_real_phases(ctx, seq) ? 1 : 0;
+            if (real) {
+                const int vb = tan ? fisp_real_tangent_tile_voxels(seq.max_state) : 32;
+                const int tiles = std::min(4, div_ceil(V, vb));
+                D = FispLaunch {0, tan ? fisp_real_tangent_queue_warps(seq.max_state, P, tiles)
+                                       : fisp_real_queue_warps(seq.max_state, P, tiles)};
+            } else {
+                D.warps = std::max(1, std::min(D.warps, 8));
+            }
+            keyed.push_back({Key {tan, D.config, D.warps, seq.max_state, real}, j});
         } else {
             const auto& seq = std::get<pSSFPSequence>(job.sequence);
             const int nz = int(seq.z.size());
@@ -189,7 +197,8 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
         if (fisp) {
             std::vector<kernels::FispArgs> args;
             const FispLaunch L {key.config, key.warps};
-            const int vb = g.tangent ? fisp_tangent_tile_voxels(L) : fisp_tile_voxels(L);
+            const int vb = g.real ? (g.tangent ? fisp_real_tangent_tile_voxels(g.cover) : 32)
+                                  : (g.tangent ? fisp_tangent_tile_voxels(L) : fisp_tile_voxels(L));
             for (size_t q = 0; q < js.size(); q++) {
                 const auto& job = jobs[size_t(js[q])];
                 const auto& seq = std::get<FISPSequence>(job.sequence);
@@ -363,13 +372,18 @@ void SimulationBatch::Impl::plan_signal(Family& fam, const std::vector<int>& mem
 void SimulationBatch::Impl::enqueue(const Family& fam, cudaStream_t stream, int* head_base) const {
     const int dev = ctx.device();
     for (const auto& g : fam.sims) {
-        if (g.fisp && g.tangent)
+        if (g.fisp && g.tangent && g.real)
+            launch_fisp_real_tangent_queue(stream, dev, g.warps, g.cover, as<kernels::FispArgs>(g.args),
+                                           as<int2>(g.items), g.nitems, head_base + g.head);
+        else if (g.fisp && g.tangent)
             launch_fisp_tangent_queue(stream, dev, FispLaunch {g.config, g.warps}, g.cover,
-                                      as<kernels::FispArgs>(g.args), as<int2>(g.items), g.nitems, head_base + g.head,
-                                      g.real);
+                                      as<kernels::FispArgs>(g.args), as<int2>(g.items), g.nitems, head_base + g.head);
+        else if (g.fisp && g.real)
+            launch_fisp_real_queue(stream, dev, g.warps, g.cover, as<kernels::FispArgs>(g.args), as<int2>(g.items),
+                                   g.nitems, head_base + g.head);
         else if (g.fisp)
             launch_fisp_queue(stream, dev, FispLaunch {g.config, g.warps}, g.cover, as<kernels::FispArgs>(g.args),
-                              as<int2>(g.items), g.nitems, head_base + g.head, g.real);
+                              as<int2>(g.items), g.nitems, head_base + g.head);
         else if (g.tangent)
             launch_pssfp_tangent_queue(stream, dev, PssfpLaunch {g.config}, g.cover, as<kernels::PssfpArgs>(g.args),
                                        as<int2>(g.items), g.nitems, head_base + g.head, g.real);

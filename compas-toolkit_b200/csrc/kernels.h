@@ -39,10 +39,27 @@ kernels::FispArgs fisp_args(const CompasContext& ctx, const TissueParameters& pa
                             const FISPSequence& seq, cfloat* echo, int64_t echo_stride);
 int fisp_tile_voxels(FispLaunch L);  // voxels per work item (tile) of layout L
 // persistent work-queue launch over (job, tile) items of FISP jobs that all use layout L;
-// *head must be 0 when the kernel starts. `real`: every job's phases are real
-// (fisp_sequence_real_phases), which a packed layout runs in its real-phase form.
+// *head must be 0 when the kernel starts
 void launch_fisp_queue(cudaStream_t stream, int device, FispLaunch L, int max_state, const kernels::FispArgs* jobs,
-                       const int2* items, int nitems, int* head, bool real = false);
+                       const int2* items, int nitems, int* head);
+// The form of sequences whose phases are real (fisp_real.cuh). covers: whether it can run the sequence,
+// by its states and spoiling; that the phases are real is read on the device (one simulation: the
+// kernel returns at once when they are not) or asked of fisp_sequence_real_phases (queue launches).
+// The echoes do not depend on the layout, the warps or the launch.
+bool fisp_real_covers(const FISPSequence& seq);
+int fisp_real_warps(int most, int P, int64_t tiles);  // warps per CTA for runs of `tiles` tiles
+int fisp_warps_override();                            // warps of set_fisp_override, or -1
+void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& args, bool balance, int* handoff,
+                      int handoff_capacity);
+void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& args);
+// work queues: items of tiles of 32 voxels (tangents: fisp_real_tangent_tile_voxels), W warps per CTA
+int fisp_real_queue_warps(int N, int P, int64_t tiles);
+int fisp_real_tangent_queue_warps(int N, int P, int64_t tiles);
+int fisp_real_tangent_tile_voxels(int N);
+void launch_fisp_real_queue(cudaStream_t stream, int device, int W, int max_state, const kernels::FispArgs* jobs,
+                            const int2* items, int nitems, int* head);
+void launch_fisp_real_tangent_queue(cudaStream_t stream, int device, int W, int max_state,
+                                    const kernels::FispArgs* jobs, const int2* items, int nitems, int* head);
 
 // value and T1/T2 tangents (forward mode) in one launch; L.config indexes the tangent layouts
 int fisp_tangent_config_count();
@@ -55,11 +72,9 @@ void launch_fisp_tangent(const CompasContext& ctx, const TissueParameters& param
                          FispLaunch L);
 int fisp_tangent_tile_voxels(FispLaunch L);  // voxels per work item of tangent layout L
 // work-queue launch over (job, tile) items of FISP tangent jobs (args with dT1 / dT2 set), every
-// job with max_state states; `real`: every job's phases are real, which a packed layout runs in its
-// real-phase form
+// job with max_state states
 void launch_fisp_tangent_queue(cudaStream_t stream, int device, FispLaunch L, int max_state,
-                               const kernels::FispArgs* jobs, const int2* items, int nitems, int* head,
-                               bool real = false);
+                               const kernels::FispArgs* jobs, const int2* items, int nitems, int* head);
 
 // ---- pSSFP ------------------------------------------------------------------------------
 struct PssfpLaunch {

@@ -86,6 +86,10 @@ void set_fisp_override(int config, int warps) {
     g_fisp_warps = warps;
 }
 
+int fisp_warps_override() {
+    return g_fisp_cfg.load() >= 0 ? g_fisp_warps.load() : -1;
+}
+
 void set_fisp_tangent_override(int config) {
     if (config >= fisp_tangent_config_count()) COMPAS_ERROR("FISP tangent layout index out of range");
     g_fisp_tangent_cfg = config;

@@ -1,0 +1,91 @@
+"""The real-phase form of the FISP simulation (csrc/fisp_real.cuh): sequences whose RF train and slice
+profiles are real run on real states without the off-resonance phases, one layout per state count,
+over 4 lanes when there are few (voxel, position) pairs. Sizes at the layouts' edges: state counts
+around the pair and lane boundaries, TRs around the 64-TR (32-TR) sample chunks, ragged voxel counts.
+Tolerance: the FP32 bound of the simulations, 1e-5 relative L2 against the FP64 oracle.
+"""
+import numpy as np
+import pytest
+
+import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+TOL_FP32 = 1e-5
+
+
+@pytest.fixture(scope="module")
+def cb():
+    import compas_b200
+
+    compas_b200.library()
+    return compas_b200
+
+
+@pytest.fixture(scope="module")
+def ctx(cb):
+    return cb.Context(0)
+
+
+def _case(nv, ntr, P, N, seed=1, **flags):
+    rng = np.random.default_rng([seed, N, P])
+    p = W.tissue_voxels(rng, nv, 22.4)
+    rf = W.smooth_flip_train(rng, ntr) * np.where(rng.uniform(size=ntr) < 0.3, -1.0, 1.0)  # phases 0 and π
+    rf[ntr // 2] = 0.0
+    slices = rng.uniform(0.2, 1.0, (P, ntr)) * np.where(rng.uniform(size=(P, 1)) < 0.3, -1.0, 1.0)
+    seq = W.fisp_sequence(rf, slices, 8.7e-3, 4.35e-3, 25e-3, N)
+    seq.update(flags)
+    return p, seq
+
+
+def _run(cb, ctx, p, seq):
+    params = cb.TissueParameters.from_soa(ctx, p)
+    s = cb.FispSequence.from_dict(ctx, seq)
+    t = cb.simulate_magnetization_tangents(ctx, params, s)
+    return [cb.simulate_magnetization(ctx, params, s).to_numpy()] + [t[k].to_numpy() for k in ("echos", "T1", "T2")]
+
+
+@pytest.mark.parametrize("N", [2, 3, 4, 5, 8, 9, 10, 13, 14, 16, 17, 18, 21, 22, 24, 25, 26, 32, 33, 34])
+@pytest.mark.parametrize("nv,ntr,P", [(37, 66, 3), (1, 64, 1), (33, 33, 1)])
+def test_state_counts_against_oracle(cb, ctx, oracle, N, nv, ntr, P):
+    p, seq = _case(nv, ntr, P, N)
+    value, echos, d1, d2 = _run(cb, ctx, p, seq)
+    assert oracle.rel_l2(value, oracle.fisp(p, seq)) < TOL_FP32
+    assert np.array_equal(value, echos) or N > 33  # 34 states: the general layouts
+    for got, field in ((d1, 0), (d2, 1)):
+        assert oracle.rel_l2(got, oracle.derivative_central(oracle.fisp, p, seq, field)) < TOL_FP32, field
+
+
+@pytest.mark.parametrize("flags", [dict(reps=3, TW=0.05, uf=2), dict(reps=2, TW=0.04, wait_spoil=0),
+                                   dict(reps=2, TW=0.04, inversion=0), dict(reps=2, TW=0.0, inversion=0, wait_spoil=0),
+                                   dict(reps=2, TW=0.04, inversion=0, wait_spoil=0)])
+@pytest.mark.parametrize("N", [6, 25])
+def test_repetitions_and_flags_against_oracle(cb, ctx, oracle, N, flags):
+    # the last combination precesses over the wait with transverse states alive: the general form
+    p, seq = _case(35, 41, 4, N, seed=2, **flags)
+    value, echos, d1, d2 = _run(cb, ctx, p, seq)
+    assert oracle.rel_l2(value, oracle.fisp(p, seq)) < TOL_FP32
+    assert oracle.rel_l2(echos, value) < 1e-6
+    for got, field in ((d1, 0), (d2, 1)):
+        assert oracle.rel_l2(got, oracle.derivative_central(oracle.fisp, p, seq, field)) < TOL_FP32, field
+
+
+@pytest.mark.parametrize("N,P,nv", [(8, 1, 15001), (25, 1, 15001), (13, 3, 10007), (25, 9, 10007), (4, 35, 10007)])
+def test_bits_do_not_depend_on_the_layout(cb, ctx, N, P, nv):
+    # one lane per voxel, whole tiles or the balanced split for many pairs, 4 lanes for a few of the same voxels
+    p, seq = _case(nv, 70, P, N, seed=3)
+    many = _run(cb, ctx, p, seq)
+    few = _run(cb, ctx, np.ascontiguousarray(p[:, 100:141]), seq)
+    for a, b, what in zip(many, few, ("value", "echos", "T1", "T2")):
+        assert np.array_equal(a[:, 100:141], b), what
+
+
+def test_a_voxel_without_relaxation_times_stays_alone(cb, ctx):
+    # a masked voxel (T1 = T2 = 0) is as it was in the general form: finite, and no other voxel changes
+    p, seq = _case(40, 40, 2, 25, seed=4)
+    ref = _run(cb, ctx, p, seq)[0]
+    p[0:2, 7] = 0.0
+    got = _run(cb, ctx, p, seq)[0]
+    assert np.isfinite(got).all()
+    keep = np.arange(40) != 7
+    assert np.array_equal(got[:, keep], ref[:, keep])
