@@ -161,10 +161,9 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
         } else {
             const auto& seq = std::get<pSSFPSequence>(job.sequence);
             const int nz = int(seq.z.size());
-            const PssfpLaunch L = tuned_pssfp_launch(nz, job.parameters.nvoxels);
-            const PssfpLaunch D = L.config < 0 ? pssfp_default_launch(nz, job.parameters.nvoxels) : L;
-            // jobs with real RF form their own groups, which a packed layout runs in its real-RF form
-            const int real = pssfp_config_packed(D.config) && pssfp_sequence_real_rf(ctx, seq) ? 1 : 0;
+            // jobs with real RF form their own groups, on the real-RF kernels
+            const int real = pssfp_sequence_real_rf(ctx, seq) ? 1 : 0;
+            const PssfpLaunch D = tuned_pssfp_launch(nz, job.parameters.nvoxels, real != 0);
             keyed.push_back({Key {tan, D.config, 0, nz, real}, j});
         }
     }

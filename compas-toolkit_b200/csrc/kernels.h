@@ -84,7 +84,10 @@ int pssfp_config_count();
 bool pssfp_config_info(int index, int* ZT, int* GZ);
 bool pssfp_config_packed(int index);  // two-wide layout: ZT/2 pairs of isochromats per lane
 PssfpLaunch pssfp_default_launch(int nz, int64_t nvoxels);
-PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels);
+PssfpLaunch pssfp_real_default_launch(int nz, int64_t nvoxels);
+// real: the layout of the real-RF kernels (pssfp_real.cuh), which differ from the general ones' only in
+// the default
+PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels, bool real = false);
 void launch_pssfp(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
                   const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride, PssfpLaunch L,
                   const int* skip = nullptr);

@@ -24,31 +24,31 @@
 #include "compas/compas.h"
 #include "job_args.cuh"
 #include "kernels.h"
+#include "pssfp_real.cuh"
 
 namespace compas {
 namespace kernels {
 
 // zap[0][i] = -(RF[0]/2)·γΔtRF[i] (the α/2 pulse), zap[1+t][i] = RF[t]·γΔtRF[i]
-// zap[row][i] for rows 0..nTR, and after them, at entry (nTR + 1)·nRF, the flag of a complex RF
-// axis: x = 1 when some entry has Im zap ≠ 0, else 0 (zeroed before the launch)
+// zap[row][i] for rows 0..nTR, and after them, at entry (nTR + 1)·nRF (zeroed before the launch), the
+// flag of a complex RF axis, x = 1 when some entry has Im zap ≠ 0, else 0, and y = the largest |Re zap|
 __global__ void pssfp_table_kernel(const float2* __restrict__ rf, int nTR, const float2* __restrict__ g, int nRF,
                                    float2* __restrict__ zap) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (nTR + 1) * nRF) return;
-    int row = idx / nRF, i = idx % nRF;
-    float2 th = row == 0 ? make_float2(-rf[0].x / 2.0f, -rf[0].y / 2.0f) : rf[row - 1];
-    const float2 v = cmul(th, g[i]);
-    zap[idx] = v;
-    if (v.y != 0.0f) zap[int64_t(nTR + 1) * nRF].x = 1.0f;  // every writer stores the same value
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = idx < (nTR + 1) * nRF;
+    float2 v = make_float2(0.f, 0.f);
+    if (in) {
+        const int row = idx / nRF, i = idx % nRF;
+        const float2 th = row == 0 ? make_float2(-rf[0].x / 2.0f, -rf[0].y / 2.0f) : rf[row - 1];
+        v = cmul(th, g[i]);
+        zap[idx] = v;
+    }
+    float2* flags = zap + int64_t(nTR + 1) * nRF;
+    if (v.y != 0.0f) flags->x = 1.0f;  // every writer stores the same value
+    // non-negative floats order as their bits (a NaN above all of them)
+    const int most = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(v.x)));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(&flags->y), most);
 }
-
-// True when every RF sample of the sequence is real (Im zap = 0: a real RF train, as with 0-π phase
-// cycling, and a real waveform). The rotation axis then has a_y = ±0 and the packed update leaves
-// out its products (pssfp_tile_packed<…, REAL>).
-__device__ __forceinline__ bool pssfp_real_rf(const PssfpArgs& a) {
-    return __ldg(&a.zap[int64_t(a.nTR + 1) * a.nRF].x) == 0.0f;
-}
-
 
 struct Iso {
     float x, y, z;
@@ -122,31 +122,27 @@ __device__ __forceinline__ float precess_angle(const PssfpArgs& a, float g, floa
 // rotation coefficients and E1 enters as E1/E2 on the E2-scaled longitudinal result. Every
 // operation is written out (no contraction left to the compiler), in the form the packed update
 // repeats on pairs of isochromats, so both give the same bits.
-// REAL (a_y = ±0, pssfp_real_rf): the products with a_y are left out, as in the packed update; the
-// same bits up to the sign of an exact zero.
-template<bool REAL = false>
 __device__ __forceinline__ void rotate_relax(Iso& m, float ax, float ay, float az, const RotCoefs& q,
                                              const RotRelax& k) {
-    const float cx = REAL ? (-az) * m.y : fmaf(ay, m.z, (-az) * m.y);
+    const float cx = fmaf(ay, m.z, (-az) * m.y);
     const float cy = fmaf(az, m.x, (-ax) * m.z);
-    const float cz = REAL ? ax * m.y : fmaf(ax, m.y, (-ay) * m.x);
-    const float hd = REAL ? q.h * fmaf(ax, m.x, az * m.z) : q.h * fmaf(ax, m.x, fmaf(ay, m.y, az * m.z));
+    const float cz = fmaf(ax, m.y, (-ay) * m.x);
+    const float hd = q.h * fmaf(ax, m.x, fmaf(ay, m.y, az * m.z));
     m.x = fmaf(q.c, m.x, fmaf(q.s, cx, hd * ax));
-    m.y = REAL ? fmaf(q.c, m.y, q.s * cy) : fmaf(q.c, m.y, fmaf(q.s, cy, hd * ay));
+    m.y = fmaf(q.c, m.y, fmaf(q.s, cy, hd * ay));
     m.z = fmaf(k.r, fmaf(q.c, m.z, fmaf(q.s, cz, hd * az)), k.oneE1);
 }
 
 // Tangent of rotate_relax: the same linear map applied to d (without the regrowth 1 - E1) plus
 // the explicit derivative (px, py, pz) of the step at the current state.
-template<bool REAL = false>
 __device__ __forceinline__ void rotate_relax_tangent(Iso& d, float ax, float ay, float az, const RotCoefs& q,
                                                      const RotRelax& k, float px, float py, float pz) {
-    const float cx = REAL ? (-az) * d.y : fmaf(ay, d.z, (-az) * d.y);
+    const float cx = fmaf(ay, d.z, (-az) * d.y);
     const float cy = fmaf(az, d.x, (-ax) * d.z);
-    const float cz = REAL ? ax * d.y : fmaf(ax, d.y, (-ay) * d.x);
-    const float hd = REAL ? q.h * fmaf(ax, d.x, az * d.z) : q.h * fmaf(ax, d.x, fmaf(ay, d.y, az * d.z));
+    const float cz = fmaf(ax, d.y, (-ay) * d.x);
+    const float hd = q.h * fmaf(ax, d.x, fmaf(ay, d.y, az * d.z));
     d.x = fmaf(q.c, d.x, fmaf(q.s, cx, fmaf(hd, ax, px)));
-    d.y = REAL ? fmaf(q.c, d.y, fmaf(q.s, cy, py)) : fmaf(q.c, d.y, fmaf(q.s, cy, fmaf(hd, ay, py)));
+    d.y = fmaf(q.c, d.y, fmaf(q.s, cy, fmaf(hd, ay, py)));
     d.z = fmaf(k.r, fmaf(q.c, d.z, fmaf(q.s, cz, hd * az)), pz);
 }
 
@@ -302,15 +298,11 @@ __device__ __forceinline__ void pssfp_tile(const PssfpArgs& a, const int tile) {
 // those of the scalar update in the same order, and the z sums run over the slots in the scalar
 // order, so layout (ZP pairs, GZ lanes) gives the same bits as the scalar (2·ZP, GZ), tangents (TAN)
 // included.
-// REAL (every RF sample real, pssfp_real_rf): a_y = ±0, so the products a_y·m_z in the cross product's
-// x, a_y·m_x in its z, a_y·m_y in a·m and hd·a_y in the new m_y are left out: 23 instructions per pair
-// and RF sample instead of 27 (value; the same four per tangent). An FMA that adds ±0 to a product
-// returns the rounded product, so the results are the same bits up to the sign of an exact zero.
 // EXTRA = 1: one more isochromat, slot 2·ZP, in scalar registers with the scalar update (the same
 // operations one-wide), so that an odd count per lane needs no padding slot (35 z on 4 lanes of 9
 // instead of 10). Its update follows the pairs' (before them, ptxas spilled 40 B in the value kernel
 // and 196 B in the tangent kernel; after them 4 B and 28 B).
-template<int ZP, int GZ, bool TAN = false, bool REAL = false, int EXTRA = 0>
+template<int ZP, int GZ, bool TAN = false, int EXTRA = 0>
 __device__ __forceinline__ void pssfp_tile_packed(const PssfpArgs& a, const int tile) {
     static_assert(EXTRA == 0 || EXTRA == 1, "at most one unpaired isochromat");
     constexpr int ZT = 2 * ZP + EXTRA;
@@ -402,26 +394,23 @@ __device__ __forceinline__ void pssfp_tile_packed(const PssfpArgs& a, const int 
                     sn = make_float2(q0.s, q1.s);
                     h = make_float2(q0.h, q1.h);
                 }
-                const float2 cx = REAL ? mul2(naz[p], my[p]) : fma2(AY, mz[p], mul2(naz[p], my[p]));
+                const float2 cx = fma2(AY, mz[p], mul2(naz[p], my[p]));
                 const float2 cy = fma2(az[p], mx[p], mul2(NAX, mz[p]));
-                const float2 cz = REAL ? mul2(AX, my[p]) : fma2(AX, my[p], mul2(NAY, mx[p]));
-                const float2 hd = REAL ? mul2(h, fma2(AX, mx[p], mul2(az[p], mz[p])))
-                                       : mul2(h, fma2(AX, mx[p], fma2(AY, my[p], mul2(az[p], mz[p]))));
+                const float2 cz = fma2(AX, my[p], mul2(NAY, mx[p]));
+                const float2 hd = mul2(h, fma2(AX, mx[p], fma2(AY, my[p], mul2(az[p], mz[p]))));
                 mx[p] = fma2(c, mx[p], fma2(sn, cx, mul2(hd, AX)));
-                my[p] = REAL ? fma2(c, my[p], mul2(sn, cy)) : fma2(c, my[p], fma2(sn, cy, mul2(hd, AY)));
+                my[p] = fma2(c, my[p], fma2(sn, cy, mul2(hd, AY)));
                 mz[p] = fma2(RX, fma2(c, mz[p], fma2(sn, cz, mul2(hd, az[p]))), ONE_E1X);
                 if constexpr (TAN) {
                     // the same map on the tangents plus the explicit terms at the new state:
                     // (0, 0, t/T1²·(m'_z - 1)) for T1, (t/T2²·m'_x, t/T2²·m'_y, 0) for T2
                     auto rotate = [&](float2& x, float2& yv, float2& z, float2 px, float2 py, float2 pz) {
-                        const float2 tx = REAL ? mul2(naz[p], yv) : fma2(AY, z, mul2(naz[p], yv));
+                        const float2 tx = fma2(AY, z, mul2(naz[p], yv));
                         const float2 ty = fma2(az[p], x, mul2(NAX, z));
-                        const float2 tz = REAL ? mul2(AX, yv) : fma2(AX, yv, mul2(NAY, x));
-                        const float2 td = REAL ? mul2(h, fma2(AX, x, mul2(az[p], z)))
-                                               : mul2(h, fma2(AX, x, fma2(AY, yv, mul2(az[p], z))));
+                        const float2 tz = fma2(AX, yv, mul2(NAY, x));
+                        const float2 td = mul2(h, fma2(AX, x, fma2(AY, yv, mul2(az[p], z))));
                         x = fma2(c, x, fma2(sn, tx, fma2(td, AX, px)));
-                        // REAL: fma2(td, ±0, py) is py exactly (py is a product or ±0)
-                        yv = REAL ? fma2(c, yv, fma2(sn, ty, py)) : fma2(c, yv, fma2(sn, ty, fma2(td, AY, py)));
+                        yv = fma2(c, yv, fma2(sn, ty, fma2(td, AY, py)));
                         z = fma2(RX, fma2(c, z, fma2(sn, tz, mul2(td, az[p]))), pz);
                     };
                     rotate(ax1[p], ay1[p], az1[p], bcast2(0.0f), bcast2(0.0f), mul2(S1EX, add2(mz[p], NEG1)));
@@ -430,10 +419,10 @@ __device__ __forceinline__ void pssfp_tile_packed(const PssfpArgs& a, const int 
             }
             if constexpr (EXTRA) {  // the unpaired isochromat, with the scalar update (pssfp_tile)
                 const RotCoefs q = rot_coefs(fmaf(-eaz, eaz, naxy2), rr);
-                rotate_relax<REAL>(em, ax, ay, eaz, q, rr);
+                rotate_relax(em, ax, ay, eaz, q, rr);
                 if constexpr (TAN) {
-                    rotate_relax_tangent<REAL>(ed1, ax, ay, eaz, q, rr, 0.0f, 0.0f, s1_ex * (em.z - 1.0f));
-                    rotate_relax_tangent<REAL>(ed2, ax, ay, eaz, q, rr, s2_ex * em.x, s2_ex * em.y, 0.0f);
+                    rotate_relax_tangent(ed1, ax, ay, eaz, q, rr, 0.0f, 0.0f, s1_ex * (em.z - 1.0f));
+                    rotate_relax_tangent(ed2, ax, ay, eaz, q, rr, s2_ex * em.x, s2_ex * em.y, 0.0f);
                 }
             }
         }
@@ -544,36 +533,29 @@ __device__ __forceinline__ void pssfp_tile_packed(const PssfpArgs& a, const int 
     }
 }
 
-// PACKED: ZT/2 pairs of isochromats per lane in the two-wide layout (pssfp_tile_packed). REAL: its
-// real-RF form; the host launches both forms of a packed layout back to back, each reads the table's
-// flag and the one that does not match returns at once (uniform over the grid).
-template<int ZT, int GZ, bool PACKED = false, bool REAL = false>
+// PACKED: ZT/2 pairs of isochromats per lane in the two-wide layout (pssfp_tile_packed). Sequences with
+// real RF run on the kernels of pssfp_real.cuh, launched beside these: each reads the table's flag and
+// the one that does not match returns at once (uniform over the grid).
+template<int ZT, int GZ, bool PACKED = false>
 __global__ void __launch_bounds__(128) pssfp_kernel(PssfpArgs a) {
     if (a.skip != nullptr && *a.skip != 0) return;  // uniform over the grid
-    if constexpr (PACKED) {
-        if (pssfp_real_rf(a) != REAL) return;
-        pssfp_tile_packed<ZT / 2, GZ, false, REAL, ZT % 2>(a, blockIdx.x);
-    } else {
-        pssfp_tile<ZT, GZ>(a, blockIdx.x);
-    }
+    if (pssfp_real_rf(a)) return;
+    if constexpr (PACKED) pssfp_tile_packed<ZT / 2, GZ, false, ZT % 2>(a, blockIdx.x);
+    else pssfp_tile<ZT, GZ>(a, blockIdx.x);
 }
 
 // One pSSFP simulation with its T1 and T2 tangents into a.echo, a.dT1, a.dT2.
-template<int ZT, int GZ, bool PACKED = false, bool REAL = false>
+template<int ZT, int GZ, bool PACKED = false>
 __global__ void __launch_bounds__(128) pssfp_tangent_kernel(PssfpArgs a) {
-    if constexpr (PACKED) {
-        if (pssfp_real_rf(a) != REAL) return;
-        pssfp_tile_packed<ZT / 2, GZ, true, REAL, ZT % 2>(a, blockIdx.x);
-    } else {
-        pssfp_tile<ZT, GZ, true>(a, blockIdx.x);
-    }
+    if (pssfp_real_rf(a)) return;
+    if constexpr (PACKED) pssfp_tile_packed<ZT / 2, GZ, true, ZT % 2>(a, blockIdx.x);
+    else pssfp_tile<ZT, GZ, true>(a, blockIdx.x);
 }
 
 // Persistent work-queue kernel for a batch of pSSFP simulations sharing one (ZT, GZ) layout:
 // CTAs of 128 threads take (job, tile) items, longest job first, through an atomic counter.
-// TAN: the value and T1/T2 tangents (pssfp_tangent_kernel's work). REAL: every job's RF is real (the
-// host groups jobs by their table's flag).
-template<int ZT, int GZ, bool TAN = false, bool PACKED = false, bool REAL = false>
+// TAN: the value and T1/T2 tangents (pssfp_tangent_kernel's work).
+template<int ZT, int GZ, bool TAN = false, bool PACKED = false>
 __global__ void __launch_bounds__(128) pssfp_queue_kernel(const PssfpArgs* __restrict__ jobs,
                                                           const int2* __restrict__ items, int nitems,
                                                           int* __restrict__ head) {
@@ -587,7 +569,7 @@ __global__ void __launch_bounds__(128) pssfp_queue_kernel(const PssfpArgs* __res
         const int2 w = items[it];
         if (threadIdx.x == 0) job = jobs[w.x];
         __syncthreads();
-        if constexpr (PACKED) pssfp_tile_packed<ZT / 2, GZ, TAN, REAL, ZT % 2>(job, w.y);
+        if constexpr (PACKED) pssfp_tile_packed<ZT / 2, GZ, TAN, ZT % 2>(job, w.y);
         else pssfp_tile<ZT, GZ, TAN>(job, w.y);
         __syncthreads();
     }
@@ -605,29 +587,18 @@ struct PssfpConfig {
     PssfpKernel tangent;
     PssfpQueueKernel tangent_queue;
     bool packed;  // two-wide layout (ZT/2 pairs of isochromats per lane), value and tangent kernels
-    // the real-RF forms (packed layouts, else null): fn_real and tangent_real launched beside fn and
-    // tangent, the queue forms instead of theirs for groups of real-RF jobs
-    PssfpKernel fn_real;
-    PssfpQueueKernel queue_real;
-    PssfpKernel tangent_real;
-    PssfpQueueKernel tangent_queue_real;
 };
 #define COMPAS_PSSFP(ZT, GZ)                                                                        \
     {ZT, GZ, kernels::pssfp_kernel<ZT, GZ>, kernels::pssfp_queue_kernel<ZT, GZ>,                 \
-     kernels::pssfp_tangent_kernel<ZT, GZ>, kernels::pssfp_queue_kernel<ZT, GZ, true>, false,     \
-     nullptr, nullptr, nullptr, nullptr}
+     kernels::pssfp_tangent_kernel<ZT, GZ>, kernels::pssfp_queue_kernel<ZT, GZ, true>, false}
 #define COMPAS_PSSFP_PACKED(ZT, GZ)                                                                 \
     {ZT, GZ, kernels::pssfp_kernel<ZT, GZ, true>, kernels::pssfp_queue_kernel<ZT, GZ, false, true>, \
-     kernels::pssfp_tangent_kernel<ZT, GZ, true>, kernels::pssfp_queue_kernel<ZT, GZ, true, true>, true, \
-     kernels::pssfp_kernel<ZT, GZ, true, true>, kernels::pssfp_queue_kernel<ZT, GZ, false, true, true>, \
-     kernels::pssfp_tangent_kernel<ZT, GZ, true, true>, kernels::pssfp_queue_kernel<ZT, GZ, true, true, true>}
+     kernels::pssfp_tangent_kernel<ZT, GZ, true>, kernels::pssfp_queue_kernel<ZT, GZ, true, true>, true}
 // packed value kernels with the scalar tangent kernels (the same bits; for layouts whose three packed
 // vectors would not fit the registers)
 #define COMPAS_PSSFP_PACKED_VALUE(ZT, GZ)                                                           \
     {ZT, GZ, kernels::pssfp_kernel<ZT, GZ, true>, kernels::pssfp_queue_kernel<ZT, GZ, false, true>, \
-     kernels::pssfp_tangent_kernel<ZT, GZ>, kernels::pssfp_queue_kernel<ZT, GZ, true>, true,      \
-     kernels::pssfp_kernel<ZT, GZ, true, true>, kernels::pssfp_queue_kernel<ZT, GZ, false, true, true>, \
-     nullptr, nullptr}
+     kernels::pssfp_tangent_kernel<ZT, GZ>, kernels::pssfp_queue_kernel<ZT, GZ, true>, true}
 const PssfpConfig kPssfpConfigs[] = {
     COMPAS_PSSFP(1, 1),  COMPAS_PSSFP(2, 1), COMPAS_PSSFP(4, 1),  COMPAS_PSSFP(8, 1),  COMPAS_PSSFP(9, 4),
     COMPAS_PSSFP(5, 8),  COMPAS_PSSFP(3, 16), COMPAS_PSSFP(2, 32), COMPAS_PSSFP(1, 32), COMPAS_PSSFP(18, 2),
@@ -655,7 +626,7 @@ bool pssfp_config_packed(int index) {
     return index >= 0 && index < pssfp_config_count() && kPssfpConfigs[index].packed;
 }
 
-// Default pSSFP layout (from timings on B200, 320 TRs of 15 RF samples): for 3 or more z positions
+// Default layout of the general kernels (from timings on B200, 320 TRs of 15 RF samples): for 3 or more z positions
 // the two-wide layout with the fewest slots (isochromats per lane × lanes) that cover nz, at most
 // 5 pairs per lane, fewer lanes first on a tie (35 z: ZT10·GZ4 packed 9.9 ms vs 11.7 ms for the best
 // scalar layout ZT9·GZ4 at 50176 voxels; 9 z: ZT10·GZ1 packed 1.64 ms vs 2.04 ms for ZT4·GZ4 at
@@ -680,6 +651,32 @@ PssfpLaunch pssfp_default_launch(int nz, int64_t nvoxels) {
     }
     if (best < 0) best = 7;  // 2 x 32 lanes covers nz ≤ 64
     return PssfpLaunch {best};
+}
+
+// Default layout of the real-RF kernels (pssfp_real.cuh): the one with the least estimated time per RF
+// sample, in cycles. A warp with ZT isochromats per lane needs 155 + 21·ZT by itself and 25 + 17·ZT of its
+// scheduler when others share it, and the fullest of the 4·148 schedulers runs the whole warps that
+// fall to it. So many voxels take the fewest slots and few voxels more lanes: 35 z of 15 RF samples and 100
+// TRs, 9 isochromats on 4 lanes / 5 on 8 / 3 on 16, in us: 279 / 229 / 212 at 2500 voxels, 279 / 234 / 272
+// at 4096, 362 / 413 / 446 at 8000. On a tie the fewer slots, then the fewer lanes. At most 10
+// isochromats per lane: the tangents of more do not fit the registers.
+PssfpLaunch pssfp_real_default_launch(int nz, int64_t nvoxels) {
+    int best = -1;
+    double best_time = 0.0;
+    auto slots = [](int i) { return kPssfpConfigs[i].ZT * kPssfpConfigs[i].GZ; };
+    for (int i = 0; i < pssfp_config_count(); i++) {
+        const auto& c = kPssfpConfigs[i];
+        if (slots(i) < nz || c.ZT > 10) continue;
+        const double warps = double(nvoxels) * c.GZ / (32.0 * 4 * 148);
+        const double time = std::max(155.0 + 21.0 * c.ZT, (25.0 + 17.0 * c.ZT) * (warps < 8.0 ? std::ceil(warps) : warps));
+        const bool tie = best >= 0 && std::abs(time - best_time) < 1e-9 * time;
+        if (best < 0 || (!tie && time < best_time) ||
+            (tie && (slots(i) < slots(best) || (slots(i) == slots(best) && c.GZ < kPssfpConfigs[best].GZ)))) {
+            best = i;
+            best_time = time;
+        }
+    }
+    return best < 0 ? pssfp_default_launch(nz, nvoxels) : PssfpLaunch {best};
 }
 
 kernels::PssfpArgs pssfp_args(const CompasContext& ctx, const TissueParameters& params, int voxel_begin,
@@ -745,6 +742,9 @@ const PssfpConfig& checked_config(PssfpLaunch L, int nz) {
     return cfg;
 }
 constexpr int kPssfpThreads = 128;
+unsigned pssfp_grid(int nvoxels, int GZ) {
+    return unsigned((int64_t(nvoxels) * GZ + kPssfpThreads - 1) / kPssfpThreads);
+}
 }  // namespace
 
 int pssfp_tile_voxels(PssfpLaunch L) {
@@ -760,22 +760,21 @@ void launch_pssfp(const CompasContext& ctx, const TissueParameters& params, int 
     if (nvoxels <= 0) return;
     if (L.config < 0) L = pssfp_default_launch(nz, nvoxels);
     const auto& cfg = checked_config(L, nz);
-    const int64_t total = int64_t(nvoxels) * cfg.GZ;
     DeviceGuard guard(ctx.device());
-    const unsigned grid = unsigned((total + kPssfpThreads - 1) / kPssfpThreads);
+    const unsigned grid = pssfp_grid(nvoxels, cfg.GZ);
     cfg.fn<<<grid, kPssfpThreads, 0, ctx.stream()>>>(a);
     check_launch("pssfp_kernel");
-    if (cfg.fn_real != nullptr) {  // the form that does not match the sequence returns at once
-        cfg.fn_real<<<grid, kPssfpThreads, 0, ctx.stream()>>>(a);
-        check_launch("pssfp_kernel (real RF)");
-    }
+    // the form that does not match the sequence returns at once
+    const auto& real = checked_config(tuned_pssfp_launch(nz, nvoxels, true), nz);
+    pssfp_real_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a);
+    check_launch("pssfp_real_kernel");
 }
 
 void launch_pssfp_queue(cudaStream_t stream, int device, PssfpLaunch L, int nz, const kernels::PssfpArgs* jobs,
                         const int2* items, int nitems, int* head, bool real) {
     if (nitems <= 0) return;
     const auto& cfg = checked_config(L, nz);
-    const PssfpQueueKernel fn = real && cfg.queue_real != nullptr ? cfg.queue_real : cfg.queue;
+    const PssfpQueueKernel fn = real ? pssfp_real_kernels(cfg.ZT, cfg.GZ).queue : cfg.queue;
     DeviceGuard guard(device);
     int per_sm = 1, sms = 148;
     COMPAS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPssfpThreads, 0));
@@ -789,7 +788,8 @@ void launch_pssfp_tangent_queue(cudaStream_t stream, int device, PssfpLaunch L, 
                                 const kernels::PssfpArgs* jobs, const int2* items, int nitems, int* head, bool real) {
     if (nitems <= 0) return;
     const auto& cfg = checked_config(L, nz);
-    const PssfpQueueKernel fn = real && cfg.tangent_queue_real != nullptr ? cfg.tangent_queue_real : cfg.tangent_queue;
+    const PssfpQueueKernel fn =
+        real ? pssfp_real_tangent_kernels(cfg.ZT, cfg.GZ).queue : cfg.tangent_queue;
     DeviceGuard guard(device);
     int per_sm = 1, sms = 148;
     COMPAS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPssfpThreads, 0));
@@ -828,15 +828,13 @@ void launch_pssfp_tangent(const CompasContext& ctx, const TissueParameters& para
     const auto& cfg = checked_config(L, nz);
     a.dT1 = reinterpret_cast<float2*>(dT1);
     a.dT2 = reinterpret_cast<float2*>(dT2);
-    const int64_t total = int64_t(nvoxels) * cfg.GZ;
     DeviceGuard guard(ctx.device());
-    const unsigned grid = unsigned((total + kPssfpThreads - 1) / kPssfpThreads);
+    const unsigned grid = pssfp_grid(nvoxels, cfg.GZ);
     cfg.tangent<<<grid, kPssfpThreads, 0, ctx.stream()>>>(a);
     check_launch("pssfp_tangent_kernel");
-    if (cfg.tangent_real != nullptr) {
-        cfg.tangent_real<<<grid, kPssfpThreads, 0, ctx.stream()>>>(a);
-        check_launch("pssfp_tangent_kernel (real RF)");
-    }
+    const auto& real = checked_config(tuned_pssfp_launch(nz, nvoxels, true), nz);
+    pssfp_real_tangent_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a);
+    check_launch("pssfp_real_kernel (tangents)");
 }
 
 MagnetizationTangents simulate_magnetization_tangents(const CompasContext& context, TissueParameters parameters,

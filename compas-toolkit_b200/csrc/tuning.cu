@@ -130,7 +130,7 @@ FispLaunch tuned_fisp_launch(int N, int64_t nvoxels, int P) {
     return d;
 }
 
-PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels) {
+PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels, bool real) {
     int cfg = g_pssfp_cfg.load();
     if (cfg >= 0) {
         int ZT = 0, GZ = 0;
@@ -143,7 +143,7 @@ PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels) {
         int ZT = 0, GZ = 0;
         if (pssfp_config_info(it->second, &ZT, &GZ) && ZT * GZ >= nz) return PssfpLaunch {it->second};
     }
-    return pssfp_default_launch(nz, nvoxels);
+    return real ? pssfp_real_default_launch(nz, nvoxels) : pssfp_default_launch(nz, nvoxels);
 }
 
 void set_tc_override(int kind, int tile, int splits) {

@@ -1,0 +1,69 @@
+"""The real-RF form of the pSSFP simulation (csrc/pssfp_real.cuh): its three modes (second order, third
+order, any angle), odd and even RF sample counts, and voxels whose transverse magnetisation does not
+outlive the pulse. Tolerance: the FP32 bound of the simulations, 1e-5 relative L2 against the FP64 oracle.
+"""
+import numpy as np
+import pytest
+
+import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+TOL_FP32 = 1e-5
+
+
+@pytest.fixture(scope="module")
+def cb():
+    import compas_b200
+
+    compas_b200.library()
+    return compas_b200
+
+
+@pytest.fixture(scope="module")
+def ctx(cb):
+    return cb.Context(0)
+
+
+def _check(cb, ctx, oracle, p, seq):
+    params = cb.TissueParameters.from_soa(ctx, p)
+    s = cb.pSSFPSequence.from_dict(ctx, seq)
+    value = cb.simulate_magnetization(ctx, params, s).to_numpy()
+    assert oracle.rel_l2(value, oracle.pssfp(p, seq)) < TOL_FP32
+    t = cb.simulate_magnetization_tangents(ctx, params, s)
+    assert np.array_equal(t["echos"].to_numpy(), value)
+    for name, field in (("T1", 0), ("T2", 1)):
+        assert oracle.rel_l2(t[name].to_numpy(), oracle.derivative_central(oracle.pssfp, p, seq, field)) < TOL_FP32, name
+
+
+# largest angle of one RF sample: 40° over nrf samples (0.1 rad at 15: second order), times scale
+@pytest.mark.parametrize("nrf,scale", [(15, 1.0), (16, 1.0), (15, 2.5), (7, 1.0), (2, 1.0), (1, 1.0), (15, 8.0), (65, 1.0)])
+@pytest.mark.parametrize("nz", [1, 2, 3, 9, 35])
+def test_modes_against_oracle(cb, ctx, oracle, nrf, scale, nz):
+    rng = np.random.default_rng([nrf, nz])
+    seq = W.pssfp_sequence(rng, 19, nrf=nrf, nz=nz)
+    seq["rf"] = (seq["rf"] * scale * rng.uniform(0.5, 1.0, 19)).astype(np.complex64)
+    _check(cb, ctx, oracle, W.tissue_voxels(rng, 37, 22.4), seq)
+
+
+def test_short_relaxation_times(cb, ctx, oracle):
+    # T2 of 20 us to 1 ms beside ordinary voxels: pulses of 1 ms take up to e^-50
+    rng = np.random.default_rng(3)
+    seq = W.pssfp_sequence(rng, 19, nrf=15, nz=9)
+    p = W.tissue_voxels(rng, 130, 22.4)
+    p[1, ::7] = np.geomspace(2e-5, 1e-3, p[1, ::7].size)
+    params = cb.TissueParameters.from_soa(ctx, p)
+    got = cb.simulate_magnetization(ctx, params, cb.pSSFPSequence.from_dict(ctx, seq)).to_numpy()
+    assert np.isfinite(got).all()
+    assert oracle.rel_l2(got, oracle.pssfp(p, seq)) < TOL_FP32
+
+
+@pytest.mark.parametrize("nv", [50, 1100, 6000, 20000])
+def test_layout_choice_covers_voxel_counts(cb, ctx, oracle, nv):
+    # few voxels take more lanes each: the same echoes to FP32 rounding whatever the choice
+    rng = np.random.default_rng(4)
+    seq = W.pssfp_sequence(rng, 17, nrf=5, nz=35)
+    p = W.tissue_voxels(rng, nv, 22.4)
+    got = cb.simulate_magnetization(ctx, cb.TissueParameters.from_soa(ctx, p), cb.pSSFPSequence.from_dict(ctx, seq))
+    idx = np.arange(0, nv, max(1, nv // 40))
+    assert oracle.rel_l2(got.to_numpy()[:, idx], oracle.pssfp(p, seq, vidx=idx)) < TOL_FP32
