@@ -16,7 +16,10 @@
 // sequence (the table's second flag) and the voxel's relaxation (mode_of); angles above half a radian
 // and pulses that outlast the relaxation run sample by sample with explicit relaxation and sincos.
 //
-// Bound by the FP32 pipe. MEASURE_PSSFP
+// Bound by the FP32 pipe. 35 z, 15 RF samples: 50176 voxels, 320 TRs 4.85 ms (7.93 ms with the 24-operation
+// rotation), tangents at 100 TRs 4.0 ms (6.3); 2500 voxels, 743 TRs 1.35 ms (3.37). The loop over the samples
+// holds an even and an odd body and a third for the last sample of an odd count: with a branch in
+// the loop instead, 10 % slower.
 #pragma once
 
 #include <cstdint>

@@ -612,7 +612,7 @@ TcPlan tc_plan(int device, int nvoxels, int R, int S, int C, bool jac) {
         // tuned: at most 64 splits and at least one voxel stage each
         splits = std::min({tuning.splits, 64, std::max(1, div_ceil(std::max(nvoxels, 1), vps))});
     } else {
-        // split the voxel range over CTAs only to fill the GPU: pick the split count (≥ 16 stages
+        // split the voxel range over CTAs only to fill the GPU: pick the split count (≥ 4 stages
         // per split) whose grid leaves the least idle SM time in the last wave of one CTA per SM,
         // less 0.5 % per split for the partial tiles written and summed. (Accuracy needs no split:
         // the tensor core's FP32 accumulation error grows with the accumulated K, ~2e-4 relative
@@ -620,7 +620,7 @@ TcPlan tc_plan(int device, int nvoxels, int R, int S, int C, bool jac) {
         // every 512 K16 steps.)
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        const int max_splits = std::max(1, std::min(64, nvoxels / (16 * vps)));
+        const int max_splits = std::max(1, std::min(64, nvoxels / (4 * vps)));
         double best = -1.0;
         for (int sp = 1; sp <= max_splits; sp++) {
             const int64_t ctas = int64_t(tiles) * sp;

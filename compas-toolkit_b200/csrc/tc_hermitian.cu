@@ -449,7 +449,7 @@ int tc_hermitian_splits(int device, int nvoxels, int R, int S, int C) {
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         double best = -1.0;
-        for (int sp = 1; sp <= std::max(1, std::min(16, ptiles / 4)); sp++) {
+        for (int sp = 1; sp <= std::max(1, std::min(64, ptiles)); sp++) {
             const int64_t ctas = int64_t(vtiles) * sp;
             const int64_t waves = (ctas + sms - 1) / sms;
             const double eff = double(ctas) / double(waves * sms) - 0.002 * sp;
