@@ -35,19 +35,19 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT / "compas-toolkit_b200"))
 
 METRIC = "EPG voxel·TR/s"
-# FMA-pipe lane operations the FISP kernel executes per (voxel, slice position, TR): every state
-# slot of the layout takes 26 one-wide operations for the excitation update (24 in the real-phase
-# form of the packed layouts, without the d_re products), and every lane 56 more for the per-TR
-# coefficients, dephasing moves and sample (ncu, profiles/fisp_epg_mrstat.txt: 732 for the 26-slot
-# packed layout in the general form)
-FISP_LANE_OPS_PER_LANE = 56
+# FP32-pipe lane operations the FISP kernel executes per (voxel, slice position, TR). Real phases with at
+# most 33 states (csrc/fisp_real.cuh): 7 per state slot, an even number of slots beside state 0, and 17
+# for state 0 and the coefficients. General layouts: 26 per slot and 56 per lane for the per-TR
+# coefficients, dephasing moves and sample.
+FISP_LANE_OPS_PER_LANE, FISP_REAL_LANE_OPS = 56, 17
 
 
 def fisp_lane_ops_per_item(cb, N, V, P, real_phases):
+    if real_phases and 2 <= N <= 33:
+        return 7 * 2 * (N // 2) + FISP_REAL_LANE_OPS, f"{2 * (N // 2)} real states + state 0"
     cfg, _ = cb.fisp_launch_choice(N, V, P)
     K, G = cb.fisp_configs()[cfg]
-    per_slot = 24 if real_phases and cb.fisp_config_packed(cfg) else 26
-    return K * G * per_slot + G * FISP_LANE_OPS_PER_LANE, f"{K}x{G}{' packed' if cb.fisp_config_packed(cfg) else ''}"
+    return K * G * 26 + G * FISP_LANE_OPS_PER_LANE, f"{K}x{G}{' packed' if cb.fisp_config_packed(cfg) else ''}"
 
 
 UNIT = "voxel·TR/s"
@@ -381,18 +381,16 @@ def main():
     Vl = ve - vb  # voxels this rank simulates
     epg_flops = 86.0 * N * P * Vl * nTR
     epg_tf = epg_flops / (sim_ms / 1e3) / 1e12
-    # the FP32 work the kernel executes: FMA-pipe lane operations per (voxel, slice position, TR),
-    # measured by ncu on the packed 26-slot layout (profiles/fisp_epg_mrstat.txt: FMA pipe busy
-    # cycles x 32 lanes / (voxels x positions x TRs)); against 148 SM x 128 lanes per cycle
-    # the kernel's form: real phases (sin φ = 0 for every RF sample times slice profile, as the table
-    # kernel computes it in FP64) run the update without the d_re products
+    # the FP32 work the kernel executes, against 148 SM x 128 lanes per cycle; its form: real phases
+    # (sin φ = 0 for every RF sample times slice profile, as the table kernel computes it in FP64) run on
+    # real states
     seqd = w["seq"]
     real_phases = not np.any(np.imag(np.asarray(seqd["slices"], np.complex128)
                                      * np.asarray(seqd["rf"], np.complex128)[None, :]))
     per_item, layout = fisp_lane_ops_per_item(cb, N, Vl, P, real_phases)
     lane_ops = per_item * P * Vl * nTR
     exec_frac = lane_ops / (sim_ms / 1e3) / (148 * 128 * f_mhz * 1e6)
-    roofline = {"bound": "fp32", "kernel": "fisp_epg_kernel", "achieved": epg_tf, "peak": fp32_peak_tf,
+    roofline = {"bound": "fp32", "kernel": "fisp_real_kernel" if real_phases else "fisp_epg_kernel", "achieved": epg_tf, "peak": fp32_peak_tf,
                 "unit": "TFLOP/s", "frac": epg_tf / fp32_peak_tf,
                 "traffic": profile_traffic("fisp_epg_mrstat"),
                 "executed": {"fp32_lane_ops_per_voxel_position_tr": per_item, "layout": layout,
@@ -400,7 +398,7 @@ def main():
                              "fp32_lane_ops": lane_ops, "frac_of_fp32_peak": exec_frac},
                 "note": f"FP32 SIMT peak 148 SM x 128 lanes x 2 x {f_mhz:.0f} MHz (median SM clock under load). "
                         "achieved/frac count the reference formulation's 86·N·P flops per voxel·TR; the kernel "
-                        f"executes {24 if real_phases else 26} FP32 operations per EPG state and TR where that "
+                        f"executes {7 if real_phases else 26} FP32 operations per EPG state and TR where that "
                         "formulation has 48, so frac can pass 1. executed.frac_of_fp32_peak is the FP32 work actually "
                         "issued (FMA-pipe lane operations, two per FFMA2) over the FP32 peak. HBM is not binding "
                         "(8 B written per voxel·TR)"}

@@ -67,7 +67,9 @@ def _fisp_name(cfg):
 def tune_fisp(ctx, N, nv, P, ntr, reps, warps=(4, 5, 6, 7, 8)):
     rng = np.random.default_rng(N * 1000 + P)
     params = cb.TissueParameters.from_soa(ctx, W.tissue_voxels(rng, nv, 22.4))
-    seq = cb.FispSequence.from_dict(ctx, W.fisp_sequence(W.smooth_flip_train(rng, ntr),
+    # complex RF samples: the layouts searched are those of the general kernels
+    rf = W.smooth_flip_train(rng, ntr) * np.exp(1j * rng.uniform(-0.5, 0.5, ntr))
+    seq = cb.FispSequence.from_dict(ctx, W.fisp_sequence(rf,
                                                         W.gaussian_slice_profile(P, ntr), 8.7e-3, 4.35e-3,
                                                         25e-3, N))
     cb.set_fisp_launch(-1, -1)
@@ -91,7 +93,9 @@ def tune_fisp(ctx, N, nv, P, ntr, reps, warps=(4, 5, 6, 7, 8)):
 def tune_pssfp(ctx, nz, nv, ntr, reps):
     rng = np.random.default_rng(nz)
     params = cb.TissueParameters.from_soa(ctx, W.tissue_voxels(rng, nv, 22.4))
-    seq = cb.pSSFPSequence.from_dict(ctx, W.pssfp_sequence(rng, ntr, nrf=15, nz=nz))
+    d = W.pssfp_sequence(rng, ntr, nrf=15, nz=nz)
+    d["rf"] = (d["rf"] * np.exp(1j * rng.uniform(-0.5, 0.5, ntr))).astype(np.complex64)  # the general kernels
+    seq = cb.pSSFPSequence.from_dict(ctx, d)
     cb.set_pssfp_launch(-1)
     default = cb.pssfp_launch_choice(nz, nv)
     candidates = {default} | {cfg for cfg, (ZT, GZ) in enumerate(cb.pssfp_configs()) if nz <= ZT * GZ <= 2 * nz + 30}

@@ -11,6 +11,9 @@
 //      compas_b200_autotune.py,
 //   3. the built-in heuristic (fisp_default_launch / pssfp_default_launch / the plan functions of
 //      the tensor-core launchers).
+// The FISP and pSSFP lines are of the general kernels. Sequences with real phases or real RF run on
+// fisp_real.cuh and pssfp_real.cuh, which choose by their own rules (an explicit pSSFP override and the
+// warps of a FISP override apply to them too).
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -137,13 +140,14 @@ PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels, bool real) {
         pssfp_config_info(cfg, &ZT, &GZ);
         if (ZT * GZ >= nz) return PssfpLaunch {cfg};
     }
+    if (real) return pssfp_real_default_launch(nz, nvoxels);  // the table is of the general kernels
     const auto& t = table();
     auto it = t.pssfp.find({nz, bucket(nvoxels)});
     if (it != t.pssfp.end()) {
         int ZT = 0, GZ = 0;
         if (pssfp_config_info(it->second, &ZT, &GZ) && ZT * GZ >= nz) return PssfpLaunch {it->second};
     }
-    return real ? pssfp_real_default_launch(nz, nvoxels) : pssfp_default_launch(nz, nvoxels);
+    return pssfp_default_launch(nz, nvoxels);
 }
 
 void set_tc_override(int kind, int tile, int splits) {
