@@ -36,10 +36,10 @@ sys.path.insert(0, str(ROOT / "compas-toolkit_b200"))
 
 METRIC = "EPG voxel·TR/s"
 # FP32-pipe lane operations the FISP kernel executes per (voxel, slice position, TR). Real phases with at
-# most 33 states (csrc/fisp_real.cuh): 7 per state slot, an even number of slots beside state 0, and 17
-# for state 0 and the coefficients. General layouts: 26 per slot and 56 per lane for the per-TR
+# most 33 states (csrc/fisp_real.cuh): 7 per state slot, an even number of slots beside state 0, and 14
+# for state 0 and the coefficients (profiles/fisp_real_mrstat.txt: 182 at 25 states). General layouts: 26 per slot and 56 per lane for the per-TR
 # coefficients, dephasing moves and sample.
-FISP_LANE_OPS_PER_LANE, FISP_REAL_LANE_OPS = 56, 17
+FISP_LANE_OPS_PER_LANE, FISP_REAL_LANE_OPS = 56, 14
 
 
 def fisp_lane_ops_per_item(cb, N, V, P, real_phases):
@@ -392,7 +392,7 @@ def main():
     exec_frac = lane_ops / (sim_ms / 1e3) / (148 * 128 * f_mhz * 1e6)
     roofline = {"bound": "fp32", "kernel": "fisp_real_kernel" if real_phases else "fisp_epg_kernel", "achieved": epg_tf, "peak": fp32_peak_tf,
                 "unit": "TFLOP/s", "frac": epg_tf / fp32_peak_tf,
-                "traffic": profile_traffic("fisp_epg_mrstat"),
+                "traffic": profile_traffic("fisp_real_mrstat" if real_phases else "fisp_epg_mrstat"),
                 "executed": {"fp32_lane_ops_per_voxel_position_tr": per_item, "layout": layout,
                              "real_phase_form": real_phases,
                              "fp32_lane_ops": lane_ops, "frac_of_fp32_peak": exec_frac},

@@ -32,7 +32,7 @@ namespace compas {
 namespace kernels {
 
 // table[p][t] = {x = ½·(π/180)·|sliceprofile[p][t]·RF[t]|, cos φ, sin φ, 2x·cos φ} for p < P (the last
-// is the signed angle of a real phase, all that fisp_real.cu reads), and in the extra
+// is the signed angle of a real phase, all that fisp_real.cuh reads), and in the extra
 // row P: table[P][0].x = 1 when some entry has sin φ ≠ 0, else 0 (the row is zeroed before the launch)
 __global__ void fisp_table_kernel(const float2* __restrict__ rf, const float2* __restrict__ slices, int nTR,
                                   int P, float4* __restrict__ table) {

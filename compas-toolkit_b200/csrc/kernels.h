@@ -99,7 +99,7 @@ void launch_pssfp_tangent(const CompasContext& ctx, const TissueParameters& para
                           const pSSFPSequence& seq, cfloat* echo, cfloat* dT1, cfloat* dT2, int64_t echo_stride,
                           PssfpLaunch L);
 // work-queue launches over (job, tile) items of pSSFP jobs that all use layout L; `real`: every job's
-// RF is real (pssfp_sequence_real_rf), which a packed layout runs in its real-RF form
+// RF is real (pssfp_sequence_real_rf), which the kernels of pssfp_real.cuh run
 void launch_pssfp_tangent_queue(cudaStream_t stream, int device, PssfpLaunch L, int nz,
                                 const kernels::PssfpArgs* jobs, const int2* items, int nitems, int* head,
                                 bool real = false);
