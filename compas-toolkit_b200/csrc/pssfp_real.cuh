@@ -12,9 +12,15 @@
 // that follows it. That is 12 or 14 operations per isochromat and RF sample (K and H to second or third
 // order in θ²), 24 before. Pairs of isochromats run as two-wide FP32 instructions.
 //
-// Which order, and whether the division is safe, is decided once per warp from the largest axis of the
-// sequence (the table's second flag) and the voxel's relaxation (mode_of); angles above half a radian
-// and pulses that outlast the relaxation run sample by sample with explicit relaxation and sincos.
+// Which order, and whether the division is safe, is decided once: the order by each lane from the largest
+// axis of the sequence (the table's second flag) and its isochromats, the division by the voxel's
+// relaxation. Angles above half a radian take longer series sample by sample (and sincos above 3π/2), and a
+// voxel that a pulse outlasts by far relaxes explicitly after every sample. The warp's vote only picks the
+// cheapest of three loops that does what all its lanes need; in each of them a lane gets the same bits
+// (what it does not need enters as a factor of 1 or a highest coefficient of 0), so a voxel's echoes
+// do not depend on its neighbours. Loop 2, in us for 20000 voxels, 60 TRs of 15 samples, 9 / 35 z (with the
+// 24-operation rotation in brackets): 30 % of the voxels with T2 = 0 338 / 662 (350 / 729; no such voxel, loop
+// 0: 170 / 394), az of 1 rad at the outer z 549 / 1523 (1349 / 2810); pulses of one sample of 40° 61 / 125 (139 / 219).
 //
 // Bound by the FP32 pipe. 35 z, 15 RF samples: 50176 voxels, 320 TRs 4.85 ms (7.93 ms with the 24-operation
 // rotation), tangents at 100 TRs 4.0 ms (6.3); 2500 voxels, 743 TRs 1.35 ms (3.37). The loop over the samples
@@ -46,7 +52,13 @@ __device__ __forceinline__ T vset(float s) {
 struct RealSample {
     float nb0, nb1, nb2;  // -B·E2^-i, -B·(E1/E2)^i, -B·(E2/E1)^i, B = ±ax
     float nax2;           // -ax²
-    float E1, E2;         // the relaxation to apply after the sample (mode 2; else divided out)
+};
+
+// What a lane needs of the loop it runs in (file header)
+struct RealNeeds {
+    float k6, h6;   // highest coefficients of K and -H: those of the third order, or 0
+    float y_min;    // no short series below this -θ²: -1/4, or -inf when no sample has more
+    float E1, E2;   // the relaxation after a sample where it is not divided out, else 1
 };
 
 // sin θ/θ, (1 - cos θ)/θ², cos θ for y = -θ²
@@ -69,21 +81,56 @@ static __device__ __noinline__ RealRotation real_rotation(float y) {  // rarely 
     return q;
 }
 
+// -sin θ/θ, -(1 - cos θ)/θ², -cos θ for y = -θ² ≥ kRealSeriesMin (θ ≤ 3π/2) on an isochromat or a pair, from
+// q = sin(θ/2)/(θ/2) and the cosine of the half angle: Taylor series in y/4 (the next terms are below 3e-9
+// and 1e-9), sin θ/θ = q·cos(θ/2), (1 - cos θ)/θ² = q²/2
+constexpr float kRealSeriesMin = -22.2f;
+template<class T>
+__device__ __forceinline__ void real_series(T y, T& ns, T& nh, T& nc) {
+    const T h = vmul(vset<T>(0.25f), y);
+    T q = vfma(h, vset<T>(1.0f / 1307674368000.0f), vset<T>(1.0f / 6227020800.0f));
+    q = vfma(h, q, vset<T>(1.0f / 39916800.0f));
+    q = vfma(h, q, vset<T>(1.0f / 362880.0f));
+    q = vfma(h, q, vset<T>(1.0f / 5040.0f));
+    q = vfma(h, q, vset<T>(1.0f / 120.0f));
+    q = vfma(h, q, vset<T>(1.0f / 6.0f));
+    q = vfma(h, q, vset<T>(1.0f));
+    T c = vfma(h, vset<T>(1.0f / 20922789888000.0f), vset<T>(1.0f / 87178291200.0f));
+    c = vfma(h, c, vset<T>(1.0f / 479001600.0f));
+    c = vfma(h, c, vset<T>(1.0f / 3628800.0f));
+    c = vfma(h, c, vset<T>(1.0f / 40320.0f));
+    c = vfma(h, c, vset<T>(1.0f / 720.0f));
+    c = vfma(h, c, vset<T>(1.0f / 24.0f));
+    c = vfma(h, c, vset<T>(0.5f));
+    c = vfma(h, c, vset<T>(1.0f));
+    const T nhq = vmul(vset<T>(-0.5f), q);
+    ns = vmul(vmul(vset<T>(-1.0f), q), c);
+    nh = vmul(nhq, q);
+    nc = vfma(y, nh, vset<T>(-1.0f));
+}
+
 // One RF sample on one isochromat or pair: x, s, z the value, (x1, s1, z1) and (x2, s2, z2) its tangents
 // ∂/∂T1, ∂/∂T2 (TAN), A = ±az, nA = -A. t1 = dt/T1², t2 = dt/T2².
-// MODE 0: θ² ≤ 0.02, 1: θ² ≤ 0.25 (the dropped terms of K and H are below 1e-8 and 1e-9), 2: any angle.
-template<int MODE, bool TAN, class T>
-__device__ __forceinline__ void real_step(T (&v)[TAN ? 9 : 3], T A, T nA, const RealSample& f, float t1, float t2) {
+// LOOP 0: θ² ≤ 0.02, 1: θ² ≤ 0.25 (the dropped terms of K and H are below 1e-8 and 1e-9), 2: any angle and
+// relaxation.
+template<int LOOP, bool TAN, class T>
+__device__ __forceinline__ void real_step(T (&v)[TAN ? 9 : 3], T A, T nA, const RealSample& f, const RealNeeds& need,
+                                          float t1, float t2) {
     const T y = vfma(nA, A, vset<T>(f.nax2));  // -θ²
     const T nb0 = vset<T>(f.nb0), nb1 = vset<T>(f.nb1), nb2 = vset<T>(f.nb2);
-    if constexpr (MODE < 2) {
+    bool taylor = true;
+    if constexpr (LOOP == 2) {
+        if constexpr (sizeof(T) == 4) taylor = y >= need.y_min;
+        else taylor = y.x >= need.y_min && y.y >= need.y_min;
+    }
+    if (taylor) {
         T K, nH;
-        if constexpr (MODE == 0) {
+        if constexpr (LOOP == 0) {
             K = vfma(y, vfma(y, vset<T>(-1.0f / 360.0f), vset<T>(1.0f / 6.0f)), vset<T>(2.0f));
             nH = vfma(y, vfma(y, vset<T>(-1.0f / 720.0f), vset<T>(-1.0f / 24.0f)), vset<T>(-0.5f));
         } else {
-            K = vfma(y, vfma(y, vfma(y, vset<T>(1.0f / 15120.0f), vset<T>(-1.0f / 360.0f)), vset<T>(1.0f / 6.0f)), vset<T>(2.0f));
-            nH = vfma(y, vfma(y, vfma(y, vset<T>(-1.0f / 40320.0f), vset<T>(-1.0f / 720.0f)), vset<T>(-1.0f / 24.0f)), vset<T>(-0.5f));
+            K = vfma(y, vfma(y, vfma(y, vset<T>(need.k6), vset<T>(-1.0f / 360.0f)), vset<T>(1.0f / 6.0f)), vset<T>(2.0f));
+            nH = vfma(y, vfma(y, vfma(y, vset<T>(need.h6), vset<T>(-1.0f / 720.0f)), vset<T>(-1.0f / 24.0f)), vset<T>(-0.5f));
         }
 #pragma unroll
         for (int q = 0; q < (TAN ? 3 : 1); q++) {
@@ -96,26 +143,39 @@ __device__ __forceinline__ void real_step(T (&v)[TAN ? 9 : 3], T A, T nA, const 
             z = vfma(nb2, u, z);
         }
     } else {
-        T S, nH, H, nS, c;
+        T nS, nH, c;
         if constexpr (sizeof(T) == 4) {
-            const RealRotation r = real_rotation(y);
-            S = r.s, H = r.h, c = -r.c;
-            nS = -S, nH = -H;
+            if (y >= kRealSeriesMin) {
+                real_series(y, nS, nH, c);
+            } else {
+                const RealRotation r = real_rotation(y);
+                nS = -r.s, nH = -r.h, c = -r.c;
+            }
         } else {
-            const RealRotation r0 = real_rotation(y.x), r1 = real_rotation(y.y);
-            S = make_float2(r0.s, r1.s), H = make_float2(r0.h, r1.h), c = make_float2(-r0.c, -r1.c);
-            nS = make_float2(-S.x, -S.y), nH = make_float2(-H.x, -H.y);
+            if (y.x >= kRealSeriesMin && y.y >= kRealSeriesMin) {
+                real_series(y, nS, nH, c);
+            } else {
+                const RealRotation r0 = real_rotation(y.x), r1 = real_rotation(y.y);
+                nS = make_float2(-r0.s, -r1.s), nH = make_float2(-r0.h, -r1.h), c = make_float2(-r0.c, -r1.c);
+            }
         }
-        (void)H;
-        const T e1 = vset<T>(f.E1), e2 = vset<T>(f.E2);
 #pragma unroll
         for (int q = 0; q < (TAN ? 3 : 1); q++) {
             T &x = v[3 * q], &s = v[3 * q + 1], &z = v[3 * q + 2];
             const T b = vfma(A, x, q == 0 ? vfma(nb1, z, nb0) : vmul(nb1, z));
             const T u = vfma(nS, s, vmul(nH, b));
-            x = vmul(e2, vfma(A, u, x));
-            s = vmul(e2, vfma(c, s, vmul(nS, b)));
-            z = vmul(e1, vfma(nb2, u, z));
+            x = vfma(A, u, x);
+            s = vfma(c, s, vmul(nS, b));
+            z = vfma(nb2, u, z);
+        }
+    }
+    if constexpr (LOOP == 2) {
+        const T e1 = vset<T>(need.E1), e2 = vset<T>(need.E2);
+#pragma unroll
+        for (int q = 0; q < (TAN ? 3 : 1); q++) {
+            v[3 * q] = vmul(e2, v[3 * q]);
+            v[3 * q + 1] = vmul(e2, v[3 * q + 1]);
+            v[3 * q + 2] = vmul(e1, v[3 * q + 2]);
         }
     }
     if constexpr (TAN) {  // the relaxation's own derivative, at the new state
@@ -201,23 +261,31 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
         for (int q = 0; q < NV; q++) O[q] = q == 2 ? z0 : q == 5 ? z0_1 : 0.f;
     }
 
-    // the warp's mode: the largest angle of any sample, and whether E1 and E2 to the power of the pulse's
-    // samples stay far from the ends of the range (a NaN fails every comparison)
+    // what the lane needs: its largest angle of any sample, and whether the voxel's E1 and E2 to the power of
+    // the pulse's samples stay far from the ends of the range (a NaN fails every comparison)
     const float zap_max = __ldg(&a.zap[int64_t(a.nTR + 1) * a.nRF].y);
     const float th2 = __fmaf_rn(zap_max * B1, zap_max * B1, azmax2);
     const float pulse = float(a.nRF) * a.dt_ex * fmaxf(fabsf(R1), fabsf(R2));
-    const bool scaled = pulse <= 40.0f && th2 <= 0.25f;
-    const int mode = !__all_sync(0xffffffffu, scaled) ? 2 : __all_sync(0xffffffffu, th2 <= 0.02f) ? 0 : 1;
+    const bool scaled = pulse <= 40.0f, second = th2 <= 0.02f, third = th2 <= 0.25f;
+    RealNeeds need;
+    need.k6 = second ? 0.0f : 1.0f / 15120.0f;
+    need.h6 = second ? 0.0f : -1.0f / 40320.0f;
+    need.y_min = third ? -INFINITY : -0.25f;
+    need.E1 = scaled ? 1.0f : E1_ex;
+    need.E2 = scaled ? 1.0f : E2_ex;
+    const int loop = !__all_sync(0xffffffffu, scaled && third) ? 2 : __all_sync(0xffffffffu, second) ? 0 : 1;
     // the pulse's decay, and the steps of the running ratios less 1 (a relaxation per sample is so close to
     // 1 that its rounding, repeated every sample, would be the largest error: as products of the factors
     // the echoes were 2e-5 off, like this 3e-6)
-    const float E1_all = mode == 2 ? 1.0f : expf(-float(a.nRF) * a.dt_ex * R1);
-    const float E2_all = mode == 2 ? 1.0f : expf(-float(a.nRF) * a.dt_ex * R2);
-    const float g0 = expm1f(a.dt_ex * R2), g1 = expm1f(a.dt_ex * __fadd_rn(R2, -R1)), g2 = expm1f(a.dt_ex * __fadd_rn(R1, -R2));
+    const float E1_all = scaled ? expf(-float(a.nRF) * a.dt_ex * R1) : 1.0f;
+    const float E2_all = scaled ? expf(-float(a.nRF) * a.dt_ex * R2) : 1.0f;
+    const float g0 = scaled ? expm1f(a.dt_ex * R2) : 0.0f;
+    const float g1 = scaled ? expm1f(a.dt_ex * __fadd_rn(R2, -R1)) : 0.0f;
+    const float g2 = scaled ? expm1f(a.dt_ex * __fadd_rn(R1, -R2)) : 0.0f;
 
     // (every lambda that touches the states is inlined by force: a call would move them to local memory)
-    auto excite = [&](int row, auto mode_tag) __attribute__((always_inline)) {
-        constexpr int MODE = decltype(mode_tag)::value;
+    auto excite = [&](int row, auto loop_tag) __attribute__((always_inline)) {
+        constexpr int LOOP = decltype(loop_tag)::value;
         const float2* zr = a.zap + int64_t(row) * a.nRF;
         float f0 = 1.f, f1 = 1.f, f2 = 1.f;
         auto sample = [&](int i, bool negative) __attribute__((always_inline)) {
@@ -228,19 +296,15 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
             f.nb1 = __fmul_rn(nb, f1);
             f.nb2 = __fmul_rn(nb, f2);
             f.nax2 = -__fmul_rn(ax, ax);
-            f.E1 = E1_ex;
-            f.E2 = E2_ex;
-            if constexpr (MODE < 2) {
-                f0 = __fmaf_rn(f0, g0, f0);
-                f1 = __fmaf_rn(f1, g1, f1);
-                f2 = __fmaf_rn(f2, g2, f2);
-            }
+            f0 = __fmaf_rn(f0, g0, f0);
+            f1 = __fmaf_rn(f1, g1, f1);
+            f2 = __fmaf_rn(f2, g2, f2);
 #pragma unroll
             for (int p = 0; p < ZP; p++) {
-                if (negative) real_step<MODE, TAN>(P[p], naz[p], az[p], f, t1_ex, t2_ex);
-                else real_step<MODE, TAN>(P[p], az[p], naz[p], f, t1_ex, t2_ex);
+                if (negative) real_step<LOOP, TAN>(P[p], naz[p], az[p], f, need, t1_ex, t2_ex);
+                else real_step<LOOP, TAN>(P[p], az[p], naz[p], f, need, t1_ex, t2_ex);
             }
-            if constexpr (ODD) real_step<MODE, TAN>(O, negative ? -oaz : oaz, negative ? oaz : -oaz, f, t1_ex, t2_ex);
+            if constexpr (ODD) real_step<LOOP, TAN>(O, negative ? -oaz : oaz, negative ? oaz : -oaz, f, need, t1_ex, t2_ex);
         };
         int i = 0;
         for (; i + 1 < a.nRF; i += 2) {
@@ -257,11 +321,6 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
             }
         }
     };
-    auto pulse_of = [&](int row) __attribute__((always_inline)) {
-        if (mode == 0) excite(row, std::integral_constant<int, 0> {});
-        else if (mode == 1) excite(row, std::integral_constant<int, 1> {});
-        else excite(row, std::integral_constant<int, 2> {});
-    };
     auto precess = [&](float E1, float E2) __attribute__((always_inline)) {
 #pragma unroll
         for (int p = 0; p < ZP; p++) real_precess<TAN>(P[p], cpr[p], spr[p], nspr[p], E1, E2, t1_pr, t2_pr);
@@ -269,54 +328,62 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
     };
     const float E1_first = E1_all * E1_pr, E2_first = E2_all * E2_pr;
 
-    // α/2 pulse, then re- and prephaser with twice the prephasing gradient (pssfp_kernels.cuh:73-80)
-    pulse_of(0);
+    // the whole sequence, once for each loop: in a common one, what the others need takes registers from
+    // loop 0 throughout (5 % of its time)
+    auto simulate = [&](auto loop_tag) __attribute__((always_inline)) {
+        auto pulse_of = [&](int row) __attribute__((always_inline)) { excite(row, loop_tag); };
+        // α/2 pulse, then re- and prephaser with twice the prephasing gradient (pssfp_kernels.cuh:73-80)
+        pulse_of(0);
 #pragma unroll
-    for (int p = 0; p < ZP; p++) {
-        float2 c, s;
-        sincosf(angle(2.0f, position(p)), &s.x, &c.x);
-        sincosf(angle(2.0f, position(p + ZP)), &s.y, &c.y);
-        real_precess<TAN>(P[p], c, s, make_float2(-s.x, -s.y), E1_first, E2_first, t1_pr, t2_pr);
-    }
-    if constexpr (ODD) {
-        float c, s;
-        sincosf(angle(2.0f, position(2 * ZP)), &s, &c);
-        real_precess<TAN>(O, c, s, -s, E1_first, E2_first, t1_pr, t2_pr);
-    }
-
-    for (int t = 0; t < a.nTR; t++) {  // pssfp_kernels.cuh:83-107
-        pulse_of(t + 1);
-        precess(E1_first, E2_first);
-        const int64_t at = int64_t(t) * a.echo_stride + a.voxel_begin + vloc;
-#pragma unroll
-        for (int q = 0; q < NV; q += 3) {
-            float sx = 0.0f, sy = 0.0f;  // over the slots in order
-#pragma unroll
-            for (int p = 0; p < ZP; p++)
-                if (sub * ZT + p < a.nz) {
-                    sx += P[p][q].x;
-                    sy += P[p][q + 1].x;
-                }
-#pragma unroll
-            for (int p = 0; p < ZP; p++)
-                if (sub * ZT + p + ZP < a.nz) {
-                    sx += P[p][q].y;
-                    sy += P[p][q + 1].y;
-                }
-            if (ODD && sub * ZT + 2 * ZP < a.nz) {
-                sx += O[q];
-                sy += O[q + 1];
-            }
-#pragma unroll
-            for (int d = GZ / 2; d > 0; d /= 2) {
-                sx += __shfl_xor_sync(0xffffffffu, sx, d, GZ);
-                sy += __shfl_xor_sync(0xffffffffu, sy, d, GZ);
-            }
-            float2* out = q == 0 ? a.echo : q == 3 ? a.dT1 : a.dT2;
-            if (sub == 0 && vok) out[at] = make_float2(sx, sy);
+        for (int p = 0; p < ZP; p++) {
+            float2 c, s;
+            sincosf(angle(2.0f, position(p)), &s.x, &c.x);
+            sincosf(angle(2.0f, position(p + ZP)), &s.y, &c.y);
+            real_precess<TAN>(P[p], c, s, make_float2(-s.x, -s.y), E1_first, E2_first, t1_pr, t2_pr);
         }
-        precess(E1_pr, E2_pr);
-    }
+        if constexpr (ODD) {
+            float c, s;
+            sincosf(angle(2.0f, position(2 * ZP)), &s, &c);
+            real_precess<TAN>(O, c, s, -s, E1_first, E2_first, t1_pr, t2_pr);
+        }
+
+        for (int t = 0; t < a.nTR; t++) {  // pssfp_kernels.cuh:83-107
+            pulse_of(t + 1);
+            precess(E1_first, E2_first);
+            const int64_t at = int64_t(t) * a.echo_stride + a.voxel_begin + vloc;
+#pragma unroll
+            for (int q = 0; q < NV; q += 3) {
+                float sx = 0.0f, sy = 0.0f;  // over the slots in order
+#pragma unroll
+                for (int p = 0; p < ZP; p++)
+                    if (sub * ZT + p < a.nz) {
+                        sx += P[p][q].x;
+                        sy += P[p][q + 1].x;
+                    }
+#pragma unroll
+                for (int p = 0; p < ZP; p++)
+                    if (sub * ZT + p + ZP < a.nz) {
+                        sx += P[p][q].y;
+                        sy += P[p][q + 1].y;
+                    }
+                if (ODD && sub * ZT + 2 * ZP < a.nz) {
+                    sx += O[q];
+                    sy += O[q + 1];
+                }
+#pragma unroll
+                for (int d = GZ / 2; d > 0; d /= 2) {
+                    sx += __shfl_xor_sync(0xffffffffu, sx, d, GZ);
+                    sy += __shfl_xor_sync(0xffffffffu, sy, d, GZ);
+                }
+                float2* out = q == 0 ? a.echo : q == 3 ? a.dT1 : a.dT2;
+                if (sub == 0 && vok) out[at] = make_float2(sx, sy);
+            }
+            precess(E1_pr, E2_pr);
+        }
+    };
+    if (loop == 0) simulate(std::integral_constant<int, 0> {});
+    else if (loop == 1) simulate(std::integral_constant<int, 1> {});
+    else simulate(std::integral_constant<int, 2> {});
 }
 
 // True when every RF sample of the sequence is real (Im zap = 0: a real RF train, as with 0-π phase

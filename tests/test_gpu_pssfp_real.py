@@ -1,6 +1,6 @@
-"""The real-RF form of the pSSFP simulation (csrc/pssfp_real.cuh): its three modes (second order, third
-order, any angle), odd and even RF sample counts, and voxels whose transverse magnetisation does not
-outlive the pulse. Tolerance: the FP32 bound of the simulations, 1e-5 relative L2 against the FP64 oracle.
+"""The real-RF form of the pSSFP simulation (csrc/pssfp_real.cuh): its three loops (second order, third
+order, any angle and relaxation), odd and even RF sample counts, voxels whose transverse magnetisation does
+not outlive the pulse, and that no voxel changes another's bits. Tolerance: the FP32 bound of the simulations, 1e-5 relative L2 against the FP64 oracle.
 """
 import numpy as np
 import pytest
@@ -46,6 +46,17 @@ def test_modes_against_oracle(cb, ctx, oracle, nrf, scale, nz):
     _check(cb, ctx, oracle, W.tissue_voxels(rng, 37, 22.4), seq)
 
 
+# one sample of 20° to 360° (B1 0.8 to 1.2): across the ends of the short series (0.5 rad), the long ones (3π/2)
+# and the half angle's sign
+@pytest.mark.parametrize("degrees", [24.0, 28.0, 29.0, 90.0, 180.0, 225.0, 260.0, 280.0, 360.0])
+@pytest.mark.parametrize("nz", [1, 9])
+def test_large_angles_against_oracle(cb, ctx, oracle, degrees, nz):
+    rng = np.random.default_rng([int(degrees), nz])
+    seq = W.pssfp_sequence(rng, 19, nrf=1, nz=nz)
+    seq["rf"] = (degrees * np.sign(seq["rf"].real)).astype(np.complex64)
+    _check(cb, ctx, oracle, W.tissue_voxels(rng, 37, 22.4), seq)
+
+
 def test_short_relaxation_times(cb, ctx, oracle):
     # T2 of 20 us to 1 ms beside ordinary voxels: pulses of 1 ms take up to e^-50
     rng = np.random.default_rng(3)
@@ -67,3 +78,41 @@ def test_layout_choice_covers_voxel_counts(cb, ctx, oracle, nv):
     got = cb.simulate_magnetization(ctx, cb.TissueParameters.from_soa(ctx, p), cb.pSSFPSequence.from_dict(ctx, seq))
     idx = np.arange(0, nv, max(1, nv // 40))
     assert oracle.rel_l2(got.to_numpy()[:, idx], oracle.pssfp(p, seq, vidx=idx)) < TOL_FP32
+
+
+@pytest.mark.parametrize("row,bad", [(1, 0.0), (1, 1e-6), (1, np.nan), (0, 0.0), (3, 5e3), (3, np.nan), (2, 40.0), (2, np.inf)])
+@pytest.mark.parametrize("nz,scale", [(1, 1.0), (9, 1.0), (35, 1.0), (9, 2.5)])
+def test_a_voxel_leaves_its_neighbours_alone(cb, ctx, row, bad, nz, scale):
+    # one voxel without relaxation times, with a NaN, or with large angles (off-resonance of 2 rad per RF
+    # sample, 40 times the flip angle) needs more than the others of its warp: their bits stay
+    rng = np.random.default_rng([nz, row])
+    seq = W.pssfp_sequence(rng, 13, nrf=15, nz=nz)
+    seq["rf"] = (seq["rf"] * scale).astype(np.complex64)
+    s = cb.pSSFPSequence.from_dict(ctx, seq)
+    nv = 45 if nz == 1 else 20001  # many voxels: several to a warp
+    p = W.tissue_voxels(rng, nv, 22.4)
+
+    def run(p):
+        params = cb.TissueParameters.from_soa(ctx, p)
+        t = cb.simulate_magnetization_tangents(ctx, params, s)
+        return [cb.simulate_magnetization(ctx, params, s).to_numpy()] + [t[k].to_numpy() for k in ("echos", "T1", "T2")]
+
+    ref = run(p)
+    p[row, 7] = bad
+    keep = np.arange(nv) != 7
+    for a, b in zip(run(p), ref):
+        assert np.array_equal(a[:, keep], b[:, keep])
+
+
+def test_large_angles_and_masked_voxels_against_oracle(cb, ctx, oracle):
+    # off-resonance of up to 1 rad per sample beside voxels on resonance and voxels with T2 = 0
+    rng = np.random.default_rng(6)
+    seq = W.pssfp_sequence(rng, 19, nrf=15, nz=9)
+    p = W.tissue_voxels(rng, 130, 22.4)
+    p[3, ::3] = rng.uniform(-2400.0, 2400.0, p[3, ::3].size)
+    _check(cb, ctx, oracle, p, seq)
+    p[1, 1::5] = 0.0
+    got = cb.simulate_magnetization(ctx, cb.TissueParameters.from_soa(ctx, p), cb.pSSFPSequence.from_dict(ctx, seq)).to_numpy()
+    assert np.array_equal(got[:, 1::5], np.zeros_like(got[:, 1::5]))
+    keep = np.arange(130) % 5 != 1
+    assert oracle.rel_l2(got[:, keep], oracle.pssfp(p[:, keep], seq)) < TOL_FP32
