@@ -66,8 +66,8 @@ void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& a, bool
     allow_smem(fn, smem);
     int grid = std::min(ntiles, resident_ctas(fn, 32 * W, smem, ctx.device()));
     // the balanced split, as for the general kernels (launch_fisp): all CTAs resident at once, and shares
-    // of at least P + W items, so that the round that publishes a CTA's tail ends before the one that
-    // waits for its predecessor's begins (a CTA waits on one other, never on a chain)
+    // of at least P + W items, which fill more than one round. (A CTA publishes its tail before it waits for its
+    // predecessor's, fisp_real_items: it waits on one other, never on a chain.)
     bool balanced = false;
     if (balance && a.P > 1 && layout->balanced != nullptr) {
         const void* bfn = reinterpret_cast<const void*>(layout->balanced);

@@ -80,6 +80,19 @@ def test_bits_do_not_depend_on_the_layout(cb, ctx, N, P, nv):
         assert np.array_equal(a[:, 100:141], b), what
 
 
+# shares of one to two tiles per CTA of the balanced split, whose tail and head fall into one round of
+# warps (12 for 25 states, 16 for 4), beside the work queue of a batch, which runs whole tiles
+@pytest.mark.parametrize("N,P,nv", [(25, 35, 6560), (25, 35, 8000), (25, 16, 9000), (4, 9, 14001), (4, 35, 8001)])
+def test_balanced_shares_below_two_tiles_match_the_queue_bits(cb, ctx, N, P, nv):
+    p, seq = _case(nv, 70, P, N, seed=5)
+    params, s = cb.TissueParameters.from_soa(ctx, p), cb.FispSequence.from_dict(ctx, seq)
+    batch = cb.SimulationBatch(ctx, [(params, s, None, None)])
+    batch.run()
+    ctx.synchronize()
+    assert np.array_equal(cb.simulate_magnetization(ctx, params, s).to_numpy(), batch.echos(0).to_numpy())
+    ctx.synchronize()  # no wait gave up
+
+
 def test_a_voxel_without_relaxation_times_stays_alone(cb, ctx):
     # a masked voxel (T1 = T2 = 0) is as it was in the general form: finite, and no other voxel changes
     p, seq = _case(40, 40, 2, 25, seed=4)
