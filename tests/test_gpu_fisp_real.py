@@ -80,6 +80,22 @@ def test_bits_do_not_depend_on_the_layout(cb, ctx, N, P, nv):
         assert np.array_equal(a[:, 100:141], b), what
 
 
+# angles past the range in which the fast sine and cosine are bounded (π), and trains whose errors of one
+# sign add up over 1000 TRs
+@pytest.mark.parametrize("train", ["5", "150", "180", "270", "360", "150-360", "5 alternating"])
+def test_flip_angles_against_oracle(cb, ctx, oracle, train):
+    p, seq = _case(37, 1000, 1, 25, seed=6)
+    lo, hi = (float(x) for x in (train.split()[0].split("-") * 2)[:2])
+    rf = np.random.default_rng(7).uniform(lo, hi, 1000)
+    if train.endswith("alternating"):
+        rf[1::2] *= -1
+    seq.update(rf=rf.astype(np.complex64), slices=np.ones((1, 1000), np.complex64))
+    value, echos, d1, d2 = _run(cb, ctx, p, seq)
+    assert oracle.rel_l2(value, oracle.fisp(p, seq)) < TOL_FP32
+    for got, field in ((d1, 0), (d2, 1)):
+        assert oracle.rel_l2(got, oracle.derivative_central(oracle.fisp, p, seq, field)) < TOL_FP32, field
+
+
 # shares of one to two tiles per CTA of the balanced split, whose tail and head fall into one round of
 # warps (12 for 25 states, 16 for 4), beside the work queue of a batch, which runs whole tiles
 @pytest.mark.parametrize("N,P,nv", [(25, 35, 6560), (25, 35, 8000), (25, 16, 9000), (4, 9, 14001), (4, 35, 8001)])
