@@ -612,26 +612,40 @@ TcPlan tc_plan(int device, int nvoxels, int R, int S, int C, bool jac) {
         // tuned: at most 64 splits and at least one voxel stage each
         splits = std::min({tuning.splits, 64, std::max(1, div_ceil(std::max(nvoxels, 1), vps))});
     } else {
-        // split the voxel range over CTAs only to fill the GPU: pick the split count (≥ 4 stages
-        // per split) whose grid leaves the least idle SM time in the last wave of one CTA per SM,
-        // less 0.5 % per split for the partial tiles written and summed (with at least 16 stages per split
-        // a 64 x 64 slice of one coil ran its signal on 32 SMs: 24 us). (Accuracy needs no split:
+        // split the voxel range over CTAs only to fill the GPU. (Accuracy needs no split:
         // the tensor core's FP32 accumulation error grows with the accumulated K, ~2e-4 relative
         // after 3750 K16 steps, measured, so each CTA folds its accumulator into an FP32 running sum
-        // every 512 K16 steps.)
+        // every 512 K16 steps.) Two rules. The coarse one: the split count (≥ 16 stages per split) whose
+        // grid leaves the least idle SM time in the last wave of one CTA per SM, less 0.5 % per split for
+        // the partial tiles written and summed. It serves all products but small ones, which it leaves on a
+        // few SMs (64 x 64 voxels, 400 readouts of one coil on 4 tiles: signal 24 us). The fine one: the least
+        // estimated time of all counts, with what was measured on 117 shapes: 0.95 us a stage, 5.2 us a CTA (its
+        // pipeline's start and the drain), and the partials' sum, 3 us, 0.1 us a split and 0.32 us/MB (so that
+        // 1000 voxels, 200 readouts of 256 samples, 16 coils keep 2 splits: J·v 67 us, with 9 89 us). It
+        // counts where the coarse grid is at most one CTA per SM and it estimates at least 5 % less.
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        const int max_splits = std::max(1, std::min(64, nvoxels / (4 * vps)));
+        const int stages = div_ceil(std::max(nvoxels, 1), vps);
+        const double mb = 8e-6 * double(C) * S * R;
+        auto waves = [&](int sp) { return double((int64_t(tiles) * sp + sms - 1) / sms); };
+        auto estimate = [&](int sp) {
+            const int per = div_ceil(stages, sp), n = div_ceil(stages, per);
+            return waves(n) * (0.95 * per + 5.2) + (n > 1 ? 3.0 + n * (0.1 + 0.32 * mb) : 0.0);
+        };
         double best = -1.0;
-        for (int sp = 1; sp <= max_splits; sp++) {
-            const int64_t ctas = int64_t(tiles) * sp;
-            const int64_t waves = (ctas + sms - 1) / sms;
-            const double eff = double(ctas) / double(waves * sms) - 0.005 * sp;
+        for (int sp = 1; sp <= std::max(1, std::min(64, nvoxels / (16 * vps))); sp++) {
+            const double eff = double(int64_t(tiles) * sp) / (waves(sp) * sms) - 0.005 * sp;
             if (eff > best + 1e-9) {
                 best = eff;
                 splits = sp;
             }
         }
+        best = waves(splits) > 1.0 ? 0.0 : 0.95 * estimate(splits);
+        for (int sp = 1; sp <= std::min(64, stages); sp++)
+            if (estimate(sp) < best - 0.005) {
+                best = estimate(sp);
+                splits = sp;
+            }
     }
     p.vchunk = std::max(vps, div_ceil(div_ceil(std::max(nvoxels, 1), splits), vps) * vps);
     p.splits = std::max(1, div_ceil(nvoxels, p.vchunk));

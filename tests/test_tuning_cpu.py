@@ -149,3 +149,28 @@ def test_tensor_core_tuning_table_is_used(tmp_path):
     assert out["cartesian_hermitian"] == [0, 5]
     assert out["spiral_signal"] == base["spiral_signal"]
     assert out["ragged"] == base["ragged"]  # 1000 readouts: log2 class 9, no line
+
+
+SPLIT_PROBE = """
+import json, sys
+sys.path.insert(0, {pkg!r})
+import compas_b200 as cb
+print(json.dumps([cb.tc_launch_choice(k, v, r, s, c)[1] for k, v, r, s, c in {shapes!r}]))
+"""
+
+
+def test_small_products_split_only_where_it_pays():
+    # (kind, voxels, readouts, samples, coils), least and most splits: products of many coils and samples, whose
+    # partial sums cost more than idle SMs, keep few splits; products on a handful of SMs are split finer
+    cases = [(("cartesian_jacobian", 1000, 200, 256, 16), 1, 3), (("cartesian_jacobian", 1000, 257, 200, 6), 1, 4),
+             (("cartesian_signal", 4096, 200, 256, 16), 1, 3), (("cartesian_signal", 2000, 1000, 48, 12), 1, 4),
+             (("cartesian_hermitian", 20000, 400, 64, 4), 1, 6), (("cartesian_hermitian", 20000, 257, 200, 6), 1, 6),
+             (("cartesian_hermitian", 7000, 743, 128, 3), 2, 5), (("cartesian_signal", 4096, 400, 64, 1), 16, 64),
+             (("cartesian_jacobian", 1000, 100, 32, 1), 8, 64), (("cartesian_hermitian", 4096, 400, 64, 1), 3, 7),
+             (("cartesian_hermitian", 500, 400, 64, 8), 25, 50)]
+    env = {k: v for k, v in os.environ.items() if k != "COMPAS_B200_TUNING"}
+    r = subprocess.run([sys.executable, "-c", SPLIT_PROBE.format(pkg=str(PKG), shapes=[c[0] for c in cases])],
+                       capture_output=True, text=True, env=env, timeout=120)
+    assert r.returncode == 0, r.stderr
+    for (shape, lo, hi), got in zip(cases, json.loads(r.stdout.strip().splitlines()[-1])):
+        assert lo <= got <= hi, (shape, got)
