@@ -86,6 +86,7 @@ struct SimulationBatch::Impl {
         bool tangent;              // value and T1/T2 tangents (tangent layouts for FISP)
         int config, warps, cover;  // layout, warps (FISP), max_state / nz
         bool real = false;         // every job's RF is real (FISP: RF and slice-profile phases)
+        bool states = false;       // FISP: on the real-state kernels
         Array<unsigned char> args;
         Array<unsigned char> items;
         int nitems = 0;
@@ -146,10 +147,12 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
                 const FispLaunch L = tuned_fisp_launch(seq.max_state, V, P);
                 D = L.config < 0 ? fisp_default_launch(seq.max_state, V, P) : L;
             }
-            // jobs with real phases form their own groups, on the real-phase kernels (an item of the
-            // queue is up to 4 tiles)
-            const int real = fisp_real_covers(seq) && fisp_sequence_real_phases(ctx, seq) ? 1 : 0;
-            if (real) {
+            // jobs with real phases form their own groups, on the real-state kernels where those cover the
+            // sequence (2; an item of the queue is up to 4 tiles), else on a packed layout's real-phase form (1)
+            const bool packed = tan ? fisp_tangent_config_packed(D.config) : fisp_config_packed(D.config);
+            const bool states = fisp_real_covers(seq);
+            const int real = (states || packed) && fisp_sequence_real_phases(ctx, seq) ? (states ? 2 : 1) : 0;
+            if (real == 2) {
                 const int vb = tan ? fisp_real_tangent_tile_voxels(seq.max_state) : 32;
                 const int tiles = std::min(4, div_ceil(V, vb));
                 D = FispLaunch {0, tan ? fisp_real_tangent_queue_warps(seq.max_state, P, tiles)
@@ -192,12 +195,13 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
         g.warps = key.warps;
         g.cover = key.cover;
         g.real = key.real != 0;
+        g.states = fisp && key.real == 2;
         std::vector<int> items;
         if (fisp) {
             std::vector<kernels::FispArgs> args;
             const FispLaunch L {key.config, key.warps};
-            const int vb = g.real ? (g.tangent ? fisp_real_tangent_tile_voxels(g.cover) : 32)
-                                  : (g.tangent ? fisp_tangent_tile_voxels(L) : fisp_tile_voxels(L));
+            const int vb = g.states ? (g.tangent ? fisp_real_tangent_tile_voxels(g.cover) : 32)
+                                    : (g.tangent ? fisp_tangent_tile_voxels(L) : fisp_tile_voxels(L));
             for (size_t q = 0; q < js.size(); q++) {
                 const auto& job = jobs[size_t(js[q])];
                 const auto& seq = std::get<FISPSequence>(job.sequence);
@@ -371,18 +375,19 @@ void SimulationBatch::Impl::plan_signal(Family& fam, const std::vector<int>& mem
 void SimulationBatch::Impl::enqueue(const Family& fam, cudaStream_t stream, int* head_base) const {
     const int dev = ctx.device();
     for (const auto& g : fam.sims) {
-        if (g.fisp && g.tangent && g.real)
+        if (g.states && g.tangent)
             launch_fisp_real_tangent_queue(stream, dev, g.warps, g.cover, as<kernels::FispArgs>(g.args),
                                            as<int2>(g.items), g.nitems, head_base + g.head);
         else if (g.fisp && g.tangent)
             launch_fisp_tangent_queue(stream, dev, FispLaunch {g.config, g.warps}, g.cover,
-                                      as<kernels::FispArgs>(g.args), as<int2>(g.items), g.nitems, head_base + g.head);
-        else if (g.fisp && g.real)
+                                      as<kernels::FispArgs>(g.args), as<int2>(g.items), g.nitems, head_base + g.head,
+                                      g.real);
+        else if (g.states)
             launch_fisp_real_queue(stream, dev, g.warps, g.cover, as<kernels::FispArgs>(g.args), as<int2>(g.items),
                                    g.nitems, head_base + g.head);
         else if (g.fisp)
             launch_fisp_queue(stream, dev, FispLaunch {g.config, g.warps}, g.cover, as<kernels::FispArgs>(g.args),
-                              as<int2>(g.items), g.nitems, head_base + g.head);
+                              as<int2>(g.items), g.nitems, head_base + g.head, g.real);
         else if (g.tangent)
             launch_pssfp_tangent_queue(stream, dev, PssfpLaunch {g.config}, g.cover, as<kernels::PssfpArgs>(g.args),
                                        as<int2>(g.items), g.nitems, head_base + g.head, g.real);

@@ -64,7 +64,7 @@ struct ExciteCoefs {
 };
 
 // Every operation is written with an explicit rounding (no multiply-add left to the compiler to
-// fuse), so that every layout gives the same bits.
+// fuse), so that the real-phase form below gives the same bits.
 __device__ __forceinline__ ExciteCoefs make_coefs(float4 tab, float B1, float2 c, float E1, float beta) {
     float s, co;
     __sincosf(tab.x * B1, &s, &co);  // x = α/2   (epg.cuh:41-51)
@@ -92,6 +92,40 @@ __device__ __forceinline__ ExciteCoefs make_coefs(float4 tab, float B1, float2 c
     k.eim = __fmaf_rn(r31re, c.y, __fmul_rn(r31im, c.x));
     k.f = __fmul_rn(ca, E1);
     k.bre = __fmul_rn(beta, r13re);
+    k.bim = __fmul_rn(beta, r13im);
+    k.bz = __fmul_rn(beta, ca);
+    return k;
+}
+
+// make_coefs for a real phase (sin φ = 0 and cos φ = ±1 exactly, as the table holds them when the
+// RF sample times the slice profile is real): cos 2φ = 1 and sin 2φ = ±0, so R12 = sin²(α/2) and
+// R13, R31 are imaginary. The products with those exact ones and zeros are left out; every other
+// operation is the general form's, so the coefficients it returns are the same bits (up to the sign
+// of an exact zero). d_re and β·R13_re, zero here, are not computed (the real-phase update does not
+// read them).
+__device__ __forceinline__ ExciteCoefs make_coefs_real(float4 tab, float B1, float2 c, float E1, float beta) {
+    float s, co;
+    __sincosf(tab.x * B1, &s, &co);
+    const float s2 = __fmul_rn(s, s), c2 = __fmul_rn(co, co);
+    const float sa = __fmul_rn(2.0f * s, co);
+    const float ca = __fmaf_rn(2.0f, c2, -1.0f);
+    const float cp = tab.y;
+    const float r13im = -__fmul_rn(cp, sa);
+    const float r31im = 0.5f * r13im;
+    const float are = __fmul_rn(c2, c.x), aim = __fmul_rn(c2, c.y);
+    const float bre = __fmul_rn(s2, c.x);
+    const float bim = -__fmul_rn(s2, c.y);
+    ExciteCoefs k;
+    k.A1 = 0.5f * __fadd_rn(are, bre);
+    k.A2 = 0.5f * __fsub_rn(bim, aim);
+    k.A3 = 0.5f * __fadd_rn(aim, bim);
+    k.A4 = 0.5f * __fsub_rn(are, bre);
+    k.dre = 0.0f;
+    k.dim = __fmul_rn(r13im, E1);
+    k.ere = -__fmul_rn(r31im, c.y);
+    k.eim = __fmul_rn(r31im, c.x);
+    k.f = __fmul_rn(ca, E1);
+    k.bre = 0.0f;
     k.bim = __fmul_rn(beta, r13im);
     k.bz = __fmul_rn(beta, ca);
     return k;
@@ -234,8 +268,9 @@ struct ExciteCoefs2 {
     float bre, bim, bz;
 };
 
+template<bool REAL = false>
 __device__ __forceinline__ ExciteCoefs2 make_coefs2(float4 tab, float B1, float2 c, float E1, float beta) {
-    const ExciteCoefs k = make_coefs(tab, B1, c, E1, beta);
+    const ExciteCoefs k = REAL ? make_coefs_real(tab, B1, c, E1, beta) : make_coefs(tab, B1, c, E1, beta);
     ExciteCoefs2 q;
     q.A1 = bcast2(k.A1);
     q.A2 = bcast2(k.A2);
@@ -328,16 +363,21 @@ struct EPGPacked {
     // excite_state on a pair with Qn = -Im Q, zn = -Im Z and nQhi = -Im Qh:
     //   Qh_r = A4·Qr + A3·Qn + d_im·zn,   -Qh_i = A2·Qr + A1·Qn + d_re·zn,
     //   Z_r' = e_re·Pr - e_im·Pi + f·Z_r,   -Z_i' = e_re·Qn - e_im·Qr + f·zn
+    // REAL (every RF phase real, fisp_real_phases): d_re and β·R13_re are ±0, so d_re·Z_r, d_re·zn and
+    // the β·R13_re additions are left out: 24 instructions per pair instead of 26. An FMA that adds ±0
+    // to a product returns the rounded product, so the results are the same bits up to the sign of an
+    // exact zero.
+    template<bool REAL = false>
     __device__ __forceinline__ void excite(const ExciteCoefs2& k, int) {
         // the unpaired slot first: the same operations one-wide (placed before the pairs, the
         // 25-slot kernel ran 44.1 ms at the MR-STAT slice; after them 45.9 ms)
         if constexpr (EXTRA) {
             const float Pr = eur + egr, Pi = eui + egi;
             const float Qr = eur - egr, Qn = egi - eui;
-            const float Phr = fmaf(k.A1.x, Pr, fmaf(k.A2.x, Pi, k.dre.x * ezr));
+            const float Phr = REAL ? fmaf(k.A1.x, Pr, k.A2.x * Pi) : fmaf(k.A1.x, Pr, fmaf(k.A2.x, Pi, k.dre.x * ezr));
             const float Phi = fmaf(k.A3.x, Pr, fmaf(k.A4.x, Pi, k.dim.x * ezr));
             const float Qhr = fmaf(k.A4.x, Qr, fmaf(k.A3.x, Qn, k.dim.x * ezn));
-            const float nQhi = fmaf(k.A2.x, Qr, fmaf(k.A1.x, Qn, k.dre.x * ezn));
+            const float nQhi = REAL ? fmaf(k.A2.x, Qr, k.A1.x * Qn) : fmaf(k.A2.x, Qr, fmaf(k.A1.x, Qn, k.dre.x * ezn));
             const float nzr = fmaf(k.ere.x, Pr, fmaf(k.neim.x, Pi, k.f.x * ezr));
             const float nzn = fmaf(k.ere.x, Qn, fmaf(k.neim.x, Qr, k.f.x * ezn));
             eur = Phr + Qhr;
@@ -351,10 +391,10 @@ struct EPGPacked {
         for (int j = 0; j < KP; j++) {
             const float2 Pr = add2(ur[j], gr[j]), Pi = add2(ui[j], gi[j]);
             const float2 Qr = sub2(ur[j], gr[j]), Qn = sub2(gi[j], ui[j]);
-            const float2 Phr = fma2(k.A1, Pr, fma2(k.A2, Pi, mul2(k.dre, zr[j])));
+            const float2 Phr = REAL ? fma2(k.A1, Pr, mul2(k.A2, Pi)) : fma2(k.A1, Pr, fma2(k.A2, Pi, mul2(k.dre, zr[j])));
             const float2 Phi = fma2(k.A3, Pr, fma2(k.A4, Pi, mul2(k.dim, zr[j])));
             const float2 Qhr = fma2(k.A4, Qr, fma2(k.A3, Qn, mul2(k.dim, zn[j])));
-            const float2 nQhi = fma2(k.A2, Qr, fma2(k.A1, Qn, mul2(k.dre, zn[j])));
+            const float2 nQhi = REAL ? fma2(k.A2, Qr, mul2(k.A1, Qn)) : fma2(k.A2, Qr, fma2(k.A1, Qn, mul2(k.dre, zn[j])));
             const float2 nzr = fma2(k.ere, Pr, fma2(k.neim, Pi, mul2(k.f, zr[j])));
             const float2 nzn = fma2(k.ere, Qn, fma2(k.neim, Qr, mul2(k.f, zn[j])));
             ur[j] = add2(Phr, Qhr);
@@ -364,8 +404,10 @@ struct EPGPacked {
             zr[j] = nzr;
             zn[j] = nzn;
         }
-        ur[0].x += k.bre;
-        gr[0].x += k.bre;
+        if constexpr (!REAL) {
+            ur[0].x += k.bre;
+            gr[0].x += k.bre;
+        }
         ui[0].x += k.bim;
         gi[0].x += k.bim;
         zr[0].x += k.bz;
@@ -529,14 +571,15 @@ struct EPGTangent {
 
 // The excitation of one pair of states in the packed representation (EPGPacked::excite's update,
 // without the regrowth terms of state 0): every operation two-wide, in excite_state's order.
+template<bool REAL>
 __device__ __forceinline__ void excite_pair(const ExciteCoefs2& k, float2& ur, float2& ui, float2& gr, float2& gi,
                                             float2& zr, float2& zn) {
     const float2 Pr = add2(ur, gr), Pi = add2(ui, gi);
     const float2 Qr = sub2(ur, gr), Qn = sub2(gi, ui);
-    const float2 Phr = fma2(k.A1, Pr, fma2(k.A2, Pi, mul2(k.dre, zr)));
+    const float2 Phr = REAL ? fma2(k.A1, Pr, mul2(k.A2, Pi)) : fma2(k.A1, Pr, fma2(k.A2, Pi, mul2(k.dre, zr)));
     const float2 Phi = fma2(k.A3, Pr, fma2(k.A4, Pi, mul2(k.dim, zr)));
     const float2 Qhr = fma2(k.A4, Qr, fma2(k.A3, Qn, mul2(k.dim, zn)));
-    const float2 nQhi = fma2(k.A2, Qr, fma2(k.A1, Qn, mul2(k.dre, zn)));
+    const float2 nQhi = REAL ? fma2(k.A2, Qr, mul2(k.A1, Qn)) : fma2(k.A2, Qr, fma2(k.A1, Qn, mul2(k.dre, zn)));
     const float2 nzr = fma2(k.ere, Pr, fma2(k.neim, Pi, mul2(k.f, zr)));
     const float2 nzn = fma2(k.ere, Qn, fma2(k.neim, Qr, mul2(k.f, zn)));
     ur = add2(Phr, Qhr);
@@ -618,6 +661,7 @@ struct EPGPackedTangent {
 
     // EPGTangent::excite: the T1 tangent excites (F1, Z1 + s1·(Z - δ_{n0})), the T2 tangent
     // (F2 + s2·F, Z2), both from the value before its own excitation
+    template<bool REAL = false>
     __device__ __forceinline__ void excite(const ExciteCoefs2& k, float s1, float s2, int sub) {
         const float2 S1 = bcast2(s1), S2 = bcast2(s2);
 #pragma unroll
@@ -626,18 +670,20 @@ struct EPGPackedTangent {
             if (j == 0 && sub == 0) zs.x = zr[0][0].x - 1.0f;
             zr[1][j] = fma2(S1, zs, zr[1][j]);
             zn[1][j] = fma2(S1, zn[0][j], zn[1][j]);
-            excite_pair(k, ur[1][j], ui[1][j], gr[1][j], gi[1][j], zr[1][j], zn[1][j]);
+            excite_pair<REAL>(k, ur[1][j], ui[1][j], gr[1][j], gi[1][j], zr[1][j], zn[1][j]);
             ur[2][j] = fma2(S2, ur[0][j], ur[2][j]);
             ui[2][j] = fma2(S2, ui[0][j], ui[2][j]);
             gr[2][j] = fma2(S2, gr[0][j], gr[2][j]);
             gi[2][j] = fma2(S2, gi[0][j], gi[2][j]);
-            excite_pair(k, ur[2][j], ui[2][j], gr[2][j], gi[2][j], zr[2][j], zn[2][j]);
+            excite_pair<REAL>(k, ur[2][j], ui[2][j], gr[2][j], gi[2][j], zr[2][j], zn[2][j]);
         }
 #pragma unroll
-        for (int j = 0; j < KP; j++) excite_pair(k, ur[0][j], ui[0][j], gr[0][j], gi[0][j], zr[0][j], zn[0][j]);
+        for (int j = 0; j < KP; j++) excite_pair<REAL>(k, ur[0][j], ui[0][j], gr[0][j], gi[0][j], zr[0][j], zn[0][j]);
         if (sub == 0) {  // the regrowth terms of state 0 (EPG::excite)
-            ur[0][0].x += k.bre;
-            gr[0][0].x += k.bre;
+            if constexpr (!REAL) {
+                ur[0][0].x += k.bre;
+                gr[0][0].x += k.bre;
+            }
             ui[0][0].x += k.bim;
             gi[0][0].x += k.bim;
             zr[0][0].x += k.bz;
@@ -751,12 +797,15 @@ using FispState =
 // tail's partial sums are published as soon as they are written and the head waits for the
 // predecessor's. Every tile's positions are still added one at a time in increasing order, so the
 // echoes are the same bits as with whole tiles per CTA.
+// REAL (packed layouts only): every RF phase is real, the excitation without the d_re products.
 // CUT0 (packed tangent layouts only): state N-1 is the first state of its lane (EPGPackedTangent).
-template<int K, int G, bool TAN = false, bool PACKED = false, bool BAL = false, bool CUT0 = false>
+template<int K, int G, bool TAN = false, bool PACKED = false, bool BAL = false, bool REAL = false,
+         bool CUT0 = false>
 __device__ __forceinline__ void fisp_items(const FispArgs& a, const int item_begin, const int item_end,
                                            float2* samples, const FispOrder* ord = nullptr) {
     static_assert(!PACKED || TAN || G == 1, "packed value layouts hold one voxel per lane");
     static_assert(!PACKED || !TAN || K % 2 == 0, "packed tangent layouts hold pairs of states");
+    static_assert(!REAL || PACKED, "the real-phase update is a packed-layout form");
     static_assert(!CUT0 || (PACKED && TAN), "the slot-0 truncation is a packed tangent form");
     constexpr int VB = 32 / G;
     const int W = blockDim.x >> 5;
@@ -847,11 +896,11 @@ __device__ __forceinline__ void fisp_items(const FispArgs& a, const int item_beg
                         if constexpr (TAN) {
                             if constexpr (PACKED) {
                                 if (t == 0) {
-                                    st.excite(make_coefs2(tv, B1, make_float2(1.f, 0.f), 1.0f, 0.0f),
+                                    st.template excite<REAL>(make_coefs2<REAL>(tv, B1, make_float2(1.f, 0.f), 1.0f, 0.0f),
                                                              0.0f, 0.0f, sub);
                                 } else {
                                     st.shift(sub, a.N);
-                                    st.excite(make_coefs2(tv, B1, c_TR, E1_TR, beta), s1_TR, s2_TR,
+                                    st.template excite<REAL>(make_coefs2<REAL>(tv, B1, c_TR, E1_TR, beta), s1_TR, s2_TR,
                                                              sub);
                                 }
                             } else {
@@ -872,10 +921,10 @@ __device__ __forceinline__ void fisp_items(const FispArgs& a, const int item_beg
                         } else {
                             if constexpr (PACKED) {
                                 if (t == 0) {
-                                    st.excite(make_coefs2(tv, B1, make_float2(1.f, 0.f), 1.0f, 0.0f), sub);
+                                    st.template excite<REAL>(make_coefs2<REAL>(tv, B1, make_float2(1.f, 0.f), 1.0f, 0.0f), sub);
                                 } else {
                                     st.shift(sub, a.N);
-                                    st.excite(make_coefs2(tv, B1, c_TR, E1_TR, beta), sub);
+                                    st.template excite<REAL>(make_coefs2<REAL>(tv, B1, c_TR, E1_TR, beta), sub);
                                 }
                             } else {
                                 if (t == 0) {
@@ -959,30 +1008,32 @@ __device__ __forceinline__ void fisp_items(const FispArgs& a, const int item_beg
 // EPGPacked<K/2> (one lane per voxel).
 // BAL instantiates the balanced form (launched with non-null `handoff`), the others the whole-tile
 // form (`handoff` unused), so that each compiles to its own register allocation.
-// A sequence that the real-phase kernels cover (a.real_form) is launched on both; each reads the
-// sequence's phase flag and the one that does not match returns at once (a branch that is uniform
-// over the grid, so no host synchronisation picks the form and the pair can be captured).
-template<int K, int G, bool PACKED = false, bool BAL = false>
+// REAL (packed layouts): the real-phase excitation. Where real phases have a kernel of their own
+// (a.real_form: the real-state kernels, or this one's REAL form for sequences that those do not cover), both
+// are launched; each reads the sequence's phase flag and the one that does not match returns at once (a branch
+// that is uniform over the grid, so no host synchronisation picks the form and the pair can be captured).
+template<int K, int G, bool PACKED = false, bool BAL = false, bool REAL = false>
 __global__ void __launch_bounds__(256, 1) fisp_epg_kernel(FispArgs a, int ntiles, int* handoff, unsigned int* status) {
     extern __shared__ float2 samples[];  // [W][32][VB]
     if (a.skip != nullptr && *a.skip != 0) return;  // uniform over the grid
-    if (a.real_form && fisp_real_phases(a)) return;
+    if (a.real_form && fisp_real_phases(a) != REAL) return;
     if constexpr (BAL) {
         __shared__ FispOrder ord;
         const int n = fisp_balanced_order(ord, ntiles, a.P, handoff, status);
-        fisp_items<K, G, false, PACKED, true>(a, 0, n, samples, &ord);
+        fisp_items<K, G, false, PACKED, true, REAL>(a, 0, n, samples, &ord);
     } else {
         (void)handoff;
         (void)status;
         const int2 r = cta_tile_range(ntiles, blockIdx.x, gridDim.x);
-        fisp_items<K, G, false, PACKED>(a, r.x * a.P, r.y * a.P, samples);
+        fisp_items<K, G, false, PACKED, false, REAL>(a, r.x * a.P, r.y * a.P, samples);
     }
 }
 
 // Persistent work-queue kernel for a batch of FISP simulations sharing one layout and W:
 // each CTA takes (job, tile) items from `items` in order through an atomic counter until the
 // queue is empty. Items are ordered longest job first, so the last wave is short.
-template<int K, int G, bool PACKED = false>
+// REAL (packed layouts): every job's phases are real, the real-phase excitation.
+template<int K, int G, bool PACKED = false, bool REAL = false>
 __global__ void __launch_bounds__(256, 1) fisp_queue_kernel(const FispArgs* __restrict__ jobs,
                                                             const int2* __restrict__ items, int nitems,
                                                             int* __restrict__ head) {
@@ -1000,25 +1051,25 @@ __global__ void __launch_bounds__(256, 1) fisp_queue_kernel(const FispArgs* __re
         // tiles w.y .. of the job, as many as the batch put in one item
         const int tiles = (job.nvoxels + 32 / G - 1) / (32 / G);
         const int t_end = min(w.y + fisp_queue_tiles_per_item(job.P, blockDim.x >> 5), tiles);
-        fisp_items<K, G, false, PACKED>(job, w.y * job.P, t_end * job.P, samples);
+        fisp_items<K, G, false, PACKED, false, REAL>(job, w.y * job.P, t_end * job.P, samples);
         __syncthreads();  // job and s_item are rewritten by the next item
     }
 }
 
 // One FISP simulation with its T1 and T2 tangents: value, ∂/∂T1, ∂/∂T2 into a.echo, a.dT1, a.dT2.
-// PACKED: the two-wide state EPGPackedTangent; CUT0 its form for (N-1) % K == 0, which the host
-// launches for those N.
-template<int K, int G, bool PACKED = false, bool CUT0 = false>
+// PACKED: the two-wide state EPGPackedTangent; REAL its real-phase form (see fisp_epg_kernel); CUT0 its
+// form for (N-1) % K == 0, which the host launches for those N.
+template<int K, int G, bool PACKED = false, bool REAL = false, bool CUT0 = false>
 __global__ void __launch_bounds__(256, 1) fisp_tangent_kernel(FispArgs a, int ntiles) {
     extern __shared__ float2 samples[];  // [3][W][chunk][VB]
-    if (a.real_form && fisp_real_phases(a)) return;
+    if (a.real_form && fisp_real_phases(a) != REAL) return;
     const int2 r = cta_tile_range(ntiles, blockIdx.x, gridDim.x);
-    fisp_items<K, G, true, PACKED, false, CUT0>(a, r.x * a.P, r.y * a.P, samples);
+    fisp_items<K, G, true, PACKED, false, REAL, CUT0>(a, r.x * a.P, r.y * a.P, samples);
 }
 
 // Work-queue form of fisp_tangent_kernel for batches (same items and order as fisp_queue_kernel;
-// CUT0: every job has (N-1) % K == 0).
-template<int K, int G, bool PACKED = false, bool CUT0 = false>
+// REAL: every job's phases are real; CUT0: every job has (N-1) % K == 0).
+template<int K, int G, bool PACKED = false, bool REAL = false, bool CUT0 = false>
 __global__ void __launch_bounds__(256, 1) fisp_tangent_queue_kernel(const FispArgs* __restrict__ jobs,
                                                                     const int2* __restrict__ items, int nitems,
                                                                     int* __restrict__ head) {
@@ -1035,7 +1086,7 @@ __global__ void __launch_bounds__(256, 1) fisp_tangent_queue_kernel(const FispAr
         __syncthreads();
         const int tiles = (job.nvoxels + 32 / G - 1) / (32 / G);
         const int t_end = min(w.y + fisp_queue_tiles_per_item(job.P, blockDim.x >> 5), tiles);
-        fisp_items<K, G, true, PACKED, false, CUT0>(job, w.y * job.P, t_end * job.P, samples);
+        fisp_items<K, G, true, PACKED, false, REAL, CUT0>(job, w.y * job.P, t_end * job.P, samples);
         __syncthreads();
     }
 }
@@ -1058,16 +1109,22 @@ struct FispConfig {
     FispValueKernel fn;
     FispQueueKernel queue;
     FispValueKernel balanced;  // the balanced item split (packed layouts), else null
+    // packed layouts: the real-phase forms of fn and balanced (launched beside them) and of queue
+    // (launched instead of it for groups of real-phase jobs), else null
+    FispValueKernel fn_real;
+    FispValueKernel balanced_real;
+    FispQueueKernel queue_real;
 };
 
 // Instantiated layouts: (states per lane K, lanes per voxel/position G). Coverage K·G ≥ N.
 // The packed one-lane layouts come last, so the indices of the others (which a tuning table
 // names) keep their meaning.
 #define COMPAS_FISP(K, G) \
-    {K, G, false, kernels::fisp_epg_kernel<K, G>, kernels::fisp_queue_kernel<K, G>, nullptr}
+    {K, G, false, kernels::fisp_epg_kernel<K, G>, kernels::fisp_queue_kernel<K, G>, nullptr, nullptr, nullptr, nullptr}
 #define COMPAS_FISP_PACKED(K)                                                                         \
     {K, 1, true, kernels::fisp_epg_kernel<K, 1, true>, kernels::fisp_queue_kernel<K, 1, true>,      \
-     kernels::fisp_epg_kernel<K, 1, true, true>}
+     kernels::fisp_epg_kernel<K, 1, true, true>, kernels::fisp_epg_kernel<K, 1, true, false, true>,  \
+     kernels::fisp_epg_kernel<K, 1, true, true, true>, kernels::fisp_queue_kernel<K, 1, true, true>}
 const FispConfig kFispConfigs[] = {
     COMPAS_FISP(1, 1), COMPAS_FISP(2, 1), COMPAS_FISP(4, 1), COMPAS_FISP(6, 1), COMPAS_FISP(8, 1),
     COMPAS_FISP(12, 1), COMPAS_FISP(16, 1), COMPAS_FISP(20, 1), COMPAS_FISP(25, 1),
@@ -1087,16 +1144,23 @@ struct FispTangentConfig {
     FispKernel fn;
     FispQueueKernel queue;
     bool packed;  // EPGPackedTangent<K/2, G>: two states per two-wide instruction
-    // packed layouts: the two kernels above in their form for (N-1) % K == 0 (state N-1 is the
+    // packed layouts: the real-phase forms of fn (launched beside it) and queue (for groups of
+    // real-phase jobs), else null
+    FispKernel fn_real;
+    FispQueueKernel queue_real;
+    // packed layouts: the four kernels above in their form for (N-1) % K == 0 (state N-1 is the
     // first state of its lane), else null
-    FispKernel fn_cut0;
-    FispQueueKernel queue_cut0;
+    FispKernel fn_cut0, fn_real_cut0;
+    FispQueueKernel queue_cut0, queue_real_cut0;
 };
-#define COMPAS_FISP_TANGENT(K, G) \
-    {K, G, kernels::fisp_tangent_kernel<K, G>, kernels::fisp_tangent_queue_kernel<K, G>, false, nullptr, nullptr}
+#define COMPAS_FISP_TANGENT(K, G)                                                                              \
+    {K, G, kernels::fisp_tangent_kernel<K, G>, kernels::fisp_tangent_queue_kernel<K, G>, false, nullptr, nullptr, \
+     nullptr, nullptr, nullptr, nullptr}
 #define COMPAS_FISP_TANGENT_PACKED(K, G)                                                                     \
     {K, G, kernels::fisp_tangent_kernel<K, G, true>, kernels::fisp_tangent_queue_kernel<K, G, true>, true, \
-     kernels::fisp_tangent_kernel<K, G, true, true>, kernels::fisp_tangent_queue_kernel<K, G, true, true>}
+     kernels::fisp_tangent_kernel<K, G, true, true>, kernels::fisp_tangent_queue_kernel<K, G, true, true>, \
+     kernels::fisp_tangent_kernel<K, G, true, false, true>, kernels::fisp_tangent_kernel<K, G, true, true, true>, \
+     kernels::fisp_tangent_queue_kernel<K, G, true, false, true>, kernels::fisp_tangent_queue_kernel<K, G, true, true, true>}
 // the packed layouts come last, so the indices of the others keep their meaning
 const FispTangentConfig kFispTangentConfigs[] = {
     COMPAS_FISP_TANGENT(1, 1), COMPAS_FISP_TANGENT(2, 1), COMPAS_FISP_TANGENT(4, 1), COMPAS_FISP_TANGENT(8, 1),
@@ -1299,43 +1363,47 @@ void launch_fisp(const CompasContext& ctx, const TissueParameters& params, int v
     if (L.config < 0) L = fisp_default_launch(N, nvoxels, P);
     kernels::FispArgs a = fisp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride);
     a.skip = skip;
-    if (fisp_real_covers(seq)) {  // this launch and the general one below: one of the two returns at once
-        launch_fisp_real(ctx, a, balance, handoff, handoff_capacity);
-        a.real_form = 1;
-    }
     const auto& cfg = checked_config(L, N);
     const int VB = 32 / cfg.G;
     const int W = std::max(1, std::min(L.warps, 8));
     const int ntiles = div_ceil(nvoxels, VB);
     const size_t smem = fisp_smem_bytes(cfg, W);
     DeviceGuard guard(ctx.device());
-    allow_smem(reinterpret_cast<const void*>(cfg.fn), smem);
-    const int grid = std::min(ntiles, resident_ctas(reinterpret_cast<const void*>(cfg.fn), 32 * W, smem, ctx.device()));
-    // The balanced split needs every CTA's share to span at least two tiles (so a CTA waits only on
-    // its predecessor's first part, never on a chain), at most kFispBalancedItems items, and all
-    // CTAs resident at once (the grid is at most one resident wave). It saves the idle tail of the
-    // CTAs with one more whole tile: 1568 tiles x 35 positions on 148 CTAs of 8 warps run 47 rounds
-    // instead of 49.
-    const int64_t per_cta = (int64_t(ntiles) * P + grid - 1) / grid;
-    bool balanced = balance && cfg.balanced != nullptr && grid > 1 && int64_t(ntiles) >= 2 * int64_t(grid) &&
-                    per_cta <= kernels::kFispBalancedItems && (handoff == nullptr || grid <= handoff_capacity);
-    if (balanced) {
-        const void* bfn = reinterpret_cast<const void*>(cfg.balanced);
-        allow_smem(bfn, smem);
-        balanced = resident_ctas(bfn, 32 * W, smem, ctx.device()) >= grid;  // every CTA resident at once
-    }
-    std::optional<Array<int, 1>> flags;
-    if (balanced) {
-        if (handoff == nullptr) {
-            flags.emplace(std::array<int64_t, 1> {grid}, ctx.device(), ctx.stream());
-            handoff = flags->data();
+    auto run = [&](FispValueKernel fn, FispValueKernel balanced_fn) {
+        allow_smem(reinterpret_cast<const void*>(fn), smem);
+        const int grid = std::min(ntiles, resident_ctas(reinterpret_cast<const void*>(fn), 32 * W, smem, ctx.device()));
+        // The balanced split needs every CTA's share to span at least two tiles (so a CTA waits only on
+        // its predecessor's first part, never on a chain), at most kFispBalancedItems items, and all
+        // CTAs resident at once (the grid is at most one resident wave). It saves the idle tail of the
+        // CTAs with one more whole tile: 1568 tiles x 35 positions on 148 CTAs of 8 warps run 47 rounds
+        // instead of 49.
+        const int64_t per_cta = (int64_t(ntiles) * P + grid - 1) / grid;
+        bool balanced = balance && balanced_fn != nullptr && grid > 1 && int64_t(ntiles) >= 2 * int64_t(grid) &&
+                        per_cta <= kernels::kFispBalancedItems && (handoff == nullptr || grid <= handoff_capacity);
+        if (balanced) {
+            const void* bfn = reinterpret_cast<const void*>(balanced_fn);
+            allow_smem(bfn, smem);
+            balanced = resident_ctas(bfn, 32 * W, smem, ctx.device()) >= grid;  // every CTA resident at once
         }
-        COMPAS_CUDA_CHECK(cudaMemsetAsync(handoff, 0, sizeof(int) * size_t(grid), ctx.stream()));
-        cfg.balanced<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles, handoff, ctx.status_word());
-    } else {
-        cfg.fn<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles, nullptr, nullptr);
-    }
-    check_launch("fisp_epg_kernel");
+        std::optional<Array<int, 1>> own;
+        int* flags = nullptr;
+        if (balanced) {
+            if (handoff == nullptr) own.emplace(std::array<int64_t, 1> {grid}, ctx.device(), ctx.stream());
+            flags = handoff == nullptr ? own->data() : handoff;
+            COMPAS_CUDA_CHECK(cudaMemsetAsync(flags, 0, sizeof(int) * size_t(grid), ctx.stream()));
+        }
+        (balanced ? balanced_fn : fn)<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles, flags, ctx.status_word());
+        check_launch("fisp_epg_kernel");
+    };
+    // real phases: on the real-state kernels, else (transverse states that live through a wait) on the real-phase
+    // form of a packed layout (24 operations per state against 26: 25 states, 9 positions, 9216 voxels, two
+    // repetitions of 150 TRs 616 us, 675 in the general form). Both forms are launched, the one that does not
+    // match the sequence returns at once.
+    const bool real_states = fisp_real_covers(seq);
+    a.real_form = real_states || cfg.fn_real != nullptr;
+    if (real_states) launch_fisp_real(ctx, a, balance, handoff, handoff_capacity);
+    else if (cfg.fn_real != nullptr) run(cfg.fn_real, cfg.balanced_real);
+    run(cfg.fn, cfg.balanced);
 }
 
 int fisp_tangent_config_count() {
@@ -1399,21 +1467,25 @@ void launch_fisp_tangent(const CompasContext& ctx, const TissueParameters& param
     COMPAS_CHECK(cfg.K * cfg.G >= N);
     a.dT1 = reinterpret_cast<float2*>(dT1);
     a.dT2 = reinterpret_cast<float2*>(dT2);
-    if (fisp_real_covers(seq)) {  // this launch and the general one below: one of the two returns at once
-        launch_fisp_real_tangent(ctx, a);
-        a.real_form = 1;
-    }
     const int VB = 32 / cfg.G;
     const int W = std::max(1, std::min(L.warps, 8));
     const int ntiles = div_ceil(nvoxels, VB);
     const size_t smem = fisp_tangent_smem_bytes(cfg.G, W);
     const bool cut0 = cfg.fn_cut0 != nullptr && (N - 1) % cfg.K == 0;
     const FispKernel fn = cut0 ? cfg.fn_cut0 : cfg.fn;
+    const FispKernel fn_real = cut0 ? cfg.fn_real_cut0 : cfg.fn_real;
     DeviceGuard guard(ctx.device());
-    allow_smem(reinterpret_cast<const void*>(fn), smem);
-    const int grid = std::min(ntiles, resident_ctas(reinterpret_cast<const void*>(fn), 32 * W, smem, ctx.device()));
-    fn<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles);
-    check_launch("fisp_tangent_kernel");
+    auto run = [&](FispKernel kernel) {
+        allow_smem(reinterpret_cast<const void*>(kernel), smem);
+        const int grid = std::min(ntiles, resident_ctas(reinterpret_cast<const void*>(kernel), 32 * W, smem, ctx.device()));
+        kernel<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles);
+        check_launch("fisp_tangent_kernel");
+    };
+    const bool real_states = fisp_real_covers(seq);  // as launch_fisp
+    a.real_form = real_states || fn_real != nullptr;
+    if (real_states) launch_fisp_real_tangent(ctx, a);
+    else if (fn_real != nullptr) run(fn_real);
+    run(fn);
 }
 
 int fisp_tangent_tile_voxels(FispLaunch L) {
@@ -1422,7 +1494,7 @@ int fisp_tangent_tile_voxels(FispLaunch L) {
 }
 
 void launch_fisp_tangent_queue(cudaStream_t stream, int device, FispLaunch L, int max_state,
-                               const kernels::FispArgs* jobs, const int2* items, int nitems, int* head) {
+                               const kernels::FispArgs* jobs, const int2* items, int nitems, int* head, bool real) {
     if (nitems <= 0) return;
     COMPAS_CHECK(L.config >= 0 && L.config < kFispTangentConfigCount);
     const auto& cfg = kFispTangentConfigs[L.config];
@@ -1430,7 +1502,8 @@ void launch_fisp_tangent_queue(cudaStream_t stream, int device, FispLaunch L, in
     // every job of the launch has max_state states (the batch groups jobs by it), so the
     // slot-0 truncation form holds for all of them or for none
     const bool cut0 = cfg.queue_cut0 != nullptr && (max_state - 1) % cfg.K == 0;
-    const FispQueueKernel fn = cut0 ? cfg.queue_cut0 : cfg.queue;
+    const bool use_real = real && cfg.queue_real != nullptr;
+    const FispQueueKernel fn = use_real ? (cut0 ? cfg.queue_real_cut0 : cfg.queue_real) : (cut0 ? cfg.queue_cut0 : cfg.queue);
     const int W = std::max(1, std::min(L.warps, 8));
     const size_t smem = fisp_tangent_smem_bytes(cfg.G, W);
     DeviceGuard guard(device);
@@ -1444,10 +1517,10 @@ void launch_fisp_tangent_queue(cudaStream_t stream, int device, FispLaunch L, in
 }
 
 void launch_fisp_queue(cudaStream_t stream, int device, FispLaunch L, int max_state, const kernels::FispArgs* jobs,
-                       const int2* items, int nitems, int* head) {
+                       const int2* items, int nitems, int* head, bool real) {
     if (nitems <= 0) return;
     const auto& cfg = checked_config(L, max_state);
-    const FispQueueKernel fn = cfg.queue;
+    const FispQueueKernel fn = real && cfg.queue_real != nullptr ? cfg.queue_real : cfg.queue;
     const int W = std::max(1, std::min(L.warps, 8));
     const size_t smem = fisp_smem_bytes(cfg, W);
     DeviceGuard guard(device);

@@ -25,7 +25,7 @@ struct FispArgs {
     float2* dT1;           // ∂echo/∂T1, ∂echo/∂T2 (same layout); used by the tangent kernels only
     float2* dT2;
     const int* skip;       // one-simulation kernel: returns at once when *skip != 0 (null: never)
-    int real_form;         // one-simulation kernel: real phases are simulated by fisp_real_kernel, return at once
+    int real_form;         // one-simulation kernels: real phases have a kernel of their own, launched beside the general one
 };
 
 // Voxel tiles per item of the FISP work-queue kernels, for a job of P slice positions on CTAs of W

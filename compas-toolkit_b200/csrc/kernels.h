@@ -39,10 +39,11 @@ kernels::FispArgs fisp_args(const CompasContext& ctx, const TissueParameters& pa
                             const FISPSequence& seq, cfloat* echo, int64_t echo_stride);
 int fisp_tile_voxels(FispLaunch L);  // voxels per work item (tile) of layout L
 // persistent work-queue launch over (job, tile) items of FISP jobs that all use layout L;
-// *head must be 0 when the kernel starts
+// *head must be 0 when the kernel starts. `real`: every job's phases are real
+// (fisp_sequence_real_phases), which a packed layout runs in its real-phase form.
 void launch_fisp_queue(cudaStream_t stream, int device, FispLaunch L, int max_state, const kernels::FispArgs* jobs,
-                       const int2* items, int nitems, int* head);
-// The form of sequences whose phases are real (fisp_real.cuh). covers: whether it can run the sequence,
+                       const int2* items, int nitems, int* head, bool real);
+// The real-state kernels of sequences whose phases are real (fisp_real.cuh). covers: whether they can run the sequence,
 // by its states and spoiling; that the phases are real is read on the device (one simulation: the
 // kernel returns at once when they are not) or asked of fisp_sequence_real_phases (queue launches).
 // The echoes do not depend on the layout, the warps or the launch.
@@ -72,9 +73,10 @@ void launch_fisp_tangent(const CompasContext& ctx, const TissueParameters& param
                          FispLaunch L);
 int fisp_tangent_tile_voxels(FispLaunch L);  // voxels per work item of tangent layout L
 // work-queue launch over (job, tile) items of FISP tangent jobs (args with dT1 / dT2 set), every
-// job with max_state states
+// job with max_state states; `real`: every job's phases are real, which a packed layout runs in its
+// real-phase form
 void launch_fisp_tangent_queue(cudaStream_t stream, int device, FispLaunch L, int max_state,
-                               const kernels::FispArgs* jobs, const int2* items, int nitems, int* head);
+                               const kernels::FispArgs* jobs, const int2* items, int nitems, int* head, bool real);
 
 // ---- pSSFP ------------------------------------------------------------------------------
 struct PssfpLaunch {

@@ -70,6 +70,27 @@ def test_repetitions_and_flags_against_oracle(cb, ctx, oracle, N, flags):
         assert oracle.rel_l2(got, oracle.derivative_central(oracle.fisp, p, seq, field)) < TOL_FP32, field
 
 
+# transverse states that live through the wait: the packed layouts' real-phase form (enough pairs for one lane
+# per voxel), alone and in a batch, beside complex phases on the general form
+@pytest.mark.parametrize("N", [8, 25, 32])
+def test_unspoiled_wait_on_packed_layouts(cb, ctx, oracle, N):
+    p, seq = _case(2500, 21, 16, N, seed=8, reps=2, TW=0.04, inversion=0, wait_spoil=0)
+    turned = dict(seq, rf=(seq["rf"] * np.exp(0.3j)).astype(np.complex64))
+    idx = np.arange(0, 2500, 60)
+    for s in (seq, turned):
+        got = _run(cb, ctx, p, s)
+        assert oracle.rel_l2(got[0][:, idx], oracle.fisp(p, s, vidx=idx)) < TOL_FP32
+        for d, field in ((got[2], 0), (got[3], 1)):
+            assert oracle.rel_l2(d[:, idx], oracle.derivative_central(oracle.fisp, p, s, field, vidx=idx)) < TOL_FP32
+        params, sequence = cb.TissueParameters.from_soa(ctx, p), cb.FispSequence.from_dict(ctx, s)
+        batch = cb.SimulationBatch(ctx, [(params, sequence, None, None)] * 2, tangents=[False, True])
+        batch.run()
+        ctx.synchronize()
+        assert np.array_equal(batch.echos(0).to_numpy(), got[0])
+        assert np.array_equal(batch.echos(1).to_numpy(), got[1])
+        assert np.array_equal(batch.derivative(1, "T1").to_numpy(), got[2])
+
+
 @pytest.mark.parametrize("N,P,nv", [(8, 1, 15001), (25, 1, 15001), (13, 3, 10007), (25, 9, 10007), (4, 35, 10007)])
 def test_bits_do_not_depend_on_the_layout(cb, ctx, N, P, nv):
     # one lane per voxel, whole tiles or the balanced split for many pairs, 4 lanes for a few of the same voxels
