@@ -876,7 +876,7 @@ def pssfp_config_packed(index: int) -> bool:
 
 
 def fisp_launch_choice(max_state: int, nvoxels: int, npositions: int) -> tuple:
-    """(layout index, warps) a FISP simulation of this shape runs with."""
+    """(layout index, warps) a FISP simulation of this shape runs with on the general kernels."""
     cfg, w = C.c_int(), C.c_int()
     library().compas_b200_fisp_launch_choice(int(max_state), int(nvoxels), int(npositions), C.byref(cfg), C.byref(w))
     return cfg.value, w.value

@@ -150,7 +150,7 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
             // jobs with real phases form their own groups, on the real-state kernels where those cover the
             // sequence (2; an item of the queue is up to 4 tiles), else on a packed layout's real-phase form (1)
             const bool packed = tan ? fisp_tangent_config_packed(D.config) : fisp_config_packed(D.config);
-            const bool states = fisp_real_covers(seq);
+            const bool states = fisp_real_covers(seq, tan != 0);
             const int real = (states || packed) && fisp_sequence_real_phases(ctx, seq) ? (states ? 2 : 1) : 0;
             if (real == 2) {
                 const int vb = tan ? fisp_real_tangent_tile_voxels(seq.max_state) : 32;

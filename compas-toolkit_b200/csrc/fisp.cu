@@ -1399,7 +1399,7 @@ void launch_fisp(const CompasContext& ctx, const TissueParameters& params, int v
     // form of a packed layout (24 operations per state against 26: 25 states, 9 positions, 9216 voxels, two
     // repetitions of 150 TRs 616 us, 675 in the general form). Both forms are launched, the one that does not
     // match the sequence returns at once.
-    const bool real_states = fisp_real_covers(seq);
+    const bool real_states = fisp_real_covers(seq, false);
     a.real_form = real_states || cfg.fn_real != nullptr;
     if (real_states) launch_fisp_real(ctx, a, balance, handoff, handoff_capacity);
     else if (cfg.fn_real != nullptr) run(cfg.fn_real, cfg.balanced_real);
@@ -1481,7 +1481,7 @@ void launch_fisp_tangent(const CompasContext& ctx, const TissueParameters& param
         kernel<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles);
         check_launch("fisp_tangent_kernel");
     };
-    const bool real_states = fisp_real_covers(seq);  // as launch_fisp
+    const bool real_states = fisp_real_covers(seq, true);  // as launch_fisp
     a.real_form = real_states || fn_real != nullptr;
     if (real_states) launch_fisp_real_tangent(ctx, a);
     else if (fn_real != nullptr) run(fn_real);

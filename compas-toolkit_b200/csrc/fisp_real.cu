@@ -36,14 +36,12 @@ const RealLayout& real_layout(int N) {
 
 }  // namespace
 
-bool fisp_real_covers(const FISPSequence& seq) {
-    return seq.max_state >= 2 && seq.max_state <= kMaxStates &&
+bool fisp_real_covers(const FISPSequence& seq, bool tangents) {
+    return seq.max_state >= 2 && seq.max_state <= kMaxStates && !fisp_layout_forced(seq.max_state, tangents) &&
            (seq.repetitions == 1 || seq.inversion_prepulse || seq.wait_spoiling || seq.TW == 0.0f);
 }
 
 int fisp_real_warps(int most, int P, int64_t tiles) {
-    const int forced = fisp_warps_override();
-    if (forced > 0) most = std::min(forced, most);
     return int(std::max<int64_t>(1, std::min<int64_t>(most, P * tiles)));
 }
 

@@ -44,12 +44,12 @@ int fisp_tile_voxels(FispLaunch L);  // voxels per work item (tile) of layout L
 void launch_fisp_queue(cudaStream_t stream, int device, FispLaunch L, int max_state, const kernels::FispArgs* jobs,
                        const int2* items, int nitems, int* head, bool real);
 // The real-state kernels of sequences whose phases are real (fisp_real.cuh). covers: whether they can run the sequence,
-// by its states and spoiling; that the phases are real is read on the device (one simulation: the
+// by its states and spoiling and by an explicit layout override; that the phases are real is read on the device (one simulation: the
 // kernel returns at once when they are not) or asked of fisp_sequence_real_phases (queue launches).
 // The echoes do not depend on the layout, the warps or the launch.
-bool fisp_real_covers(const FISPSequence& seq);
+bool fisp_real_covers(const FISPSequence& seq, bool tangents);
 int fisp_real_warps(int most, int P, int64_t tiles);  // warps per CTA for runs of `tiles` tiles
-int fisp_warps_override();                            // warps of set_fisp_override, or -1
+bool fisp_layout_forced(int N, bool tangents);        // an explicit override names a general layout that holds N states
 void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& args, bool balance, int* handoff,
                       int handoff_capacity);
 void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& args);

@@ -12,8 +12,9 @@
 //   3. the built-in heuristic (fisp_default_launch / pssfp_default_launch / the plan functions of
 //      the tensor-core launchers).
 // The FISP and pSSFP lines are of the general kernels. Sequences with real phases or real RF run on
-// fisp_real.cuh and pssfp_real.cuh, which choose by their own rules (an explicit pSSFP override and the
-// warps of a FISP override apply to them too).
+// fisp_real.cuh and pssfp_real.cuh, which choose by their own rules. An explicit FISP override that covers the
+// states means a layout of the general kernels, which then run real phases too; the pSSFP layouts are those of
+// both kernels, and an explicit override applies to either.
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -89,8 +90,10 @@ void set_fisp_override(int config, int warps) {
     g_fisp_warps = warps;
 }
 
-int fisp_warps_override() {
-    return g_fisp_cfg.load() >= 0 ? g_fisp_warps.load() : -1;
+bool fisp_layout_forced(int N, bool tangents) {
+    int K = 0, G = 0;
+    const int cfg = tangents ? g_fisp_tangent_cfg.load() : g_fisp_cfg.load();
+    return cfg >= 0 && (tangents ? fisp_tangent_config_info(cfg, &K, &G) : fisp_config_info(cfg, &K, &G)) && K * G >= N;
 }
 
 void set_fisp_tangent_override(int config) {

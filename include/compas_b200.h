@@ -197,7 +197,10 @@ COMPAS_API int compas_b200_wait_probe(const compas_context* ctx, int64_t limit_c
 COMPAS_API uint64_t compas_b200_launch_count(void);
 
 /* Launch-layout overrides used by the autotuner: FISP (config index, warps per CTA) and
- * pSSFP (config index); -1 restores the built-in choice. Number/description of layouts. */
+ * pSSFP (config index); -1 restores the built-in choice. Number/description of layouts.
+ * The FISP layouts are those of the general kernels: a sequence with real RF phases and at most 33 states,
+ * which runs on kernels of its own with their own layouts, runs on the general ones while an override
+ * that covers its states is set. The pSSFP layouts are those of the general and of the real-RF kernels. */
 COMPAS_API void compas_b200_set_fisp_launch(int config, int warps);
 COMPAS_API void compas_b200_set_pssfp_launch(int config);
 COMPAS_API int compas_b200_fisp_config_count(void);
@@ -211,15 +214,16 @@ COMPAS_API int compas_b200_pssfp_config_info(int index, int* iso_per_lane, int* 
  * lane, one two-wide FP32 instruction per pair; the same bits as the scalar layout of that size),
  * else 0. */
 COMPAS_API int compas_b200_pssfp_config_packed(int index);
-/* Layouts of the FISP tangent kernel (compas_b200_simulate_magnetization_tangents); the
- * override (-1 = built-in choice) applies when it covers the state count. */
+/* Layouts of the general FISP tangent kernel (compas_b200_simulate_magnetization_tangents); the
+ * override (-1 = built-in choice) applies when it covers the state count, to real RF phases too. */
 COMPAS_API void compas_b200_set_fisp_tangent_launch(int config);
 COMPAS_API int compas_b200_fisp_tangent_config_count(void);
 COMPAS_API int compas_b200_fisp_tangent_config_info(int index, int* states_per_lane, int* lanes);
 /* 1 when FISP tangent layout `index` is a two-wide layout (value, ∂/∂T1 and ∂/∂T2 of states_per_lane
  * states as pairs; the same bits as the scalar tangent layout of that shape), else 0. */
 COMPAS_API int compas_b200_fisp_tangent_config_packed(int index);
-/* The layout a simulation of this shape gets (override, tuning table, or built-in choice). */
+/* The layout a simulation of this shape gets on the general kernels (override, tuning table, or built-in
+ * choice). Without an override, sequences with real RF phases or real RF choose by rules of their own. */
 COMPAS_API void compas_b200_fisp_launch_choice(int max_state, int64_t nvoxels, int npositions, int* config,
                                                int* warps);
 COMPAS_API int compas_b200_pssfp_launch_choice(int nz, int64_t nvoxels);

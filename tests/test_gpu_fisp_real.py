@@ -91,6 +91,38 @@ def test_unspoiled_wait_on_packed_layouts(cb, ctx, oracle, N):
         assert np.array_equal(batch.derivative(1, "T1").to_numpy(), got[2])
 
 
+# an explicit layout override means a layout of the general kernels, for real phases too: other bits than
+# the real-state kernels' (both within FP32 of each other), the same alone and in a batch
+@pytest.mark.parametrize("tangents", [False, True])
+def test_layout_override_runs_the_general_layout(cb, ctx, oracle, tangents):
+    p, seq = _case(300, 50, 2, 8, seed=9)
+    params, s = cb.TissueParameters.from_soa(ctx, p), cb.FispSequence.from_dict(ctx, seq)
+
+    def run():
+        if not tangents:
+            return [cb.simulate_magnetization(ctx, params, s).to_numpy()]
+        t = cb.simulate_magnetization_tangents(ctx, params, s)
+        return [t[k].to_numpy() for k in ("echos", "T1", "T2")]
+
+    force = cb.set_fisp_tangent_launch if tangents else cb.set_fisp_launch
+    configs = cb.fisp_tangent_configs() if tangents else cb.fisp_configs()
+    own = run()
+    try:
+        force(next(i for i, c in enumerate(configs) if tuple(c) == (8, 1)))
+        forced = run()
+        batch = cb.SimulationBatch(ctx, [(params, s, None, None)], tangents=[tangents])
+        batch.run()
+        ctx.synchronize()
+        assert np.array_equal(batch.echos(0).to_numpy(), forced[0])
+        force(next(i for i, c in enumerate(configs) if c[0] * c[1] < 8))  # does not hold the states
+        small = run()
+    finally:
+        force(-1)
+    for a, b, c in zip(own, forced, small):
+        assert not np.array_equal(a, b) and oracle.rel_l2(b, a) < TOL_FP32
+        assert np.array_equal(a, c)
+
+
 @pytest.mark.parametrize("N,P,nv", [(8, 1, 15001), (25, 1, 15001), (13, 3, 10007), (25, 9, 10007), (4, 35, 10007)])
 def test_bits_do_not_depend_on_the_layout(cb, ctx, N, P, nv):
     # one lane per voxel, whole tiles or the balanced split for many pairs, 4 lanes for a few of the same voxels
