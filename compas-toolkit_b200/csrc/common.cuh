@@ -47,6 +47,13 @@ inline void check_launch(const char* what) {
     if (err != cudaSuccess) throw_exception(__FILE__, __LINE__, std::string(what) + ": " + cudaGetErrorString(err));
 }
 
+inline bool stream_captured(cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t err = cudaStreamIsCapturing(stream, &capture);
+    if (err != cudaSuccess) throw_exception(__FILE__, __LINE__, std::string("cudaStreamIsCapturing: ") + cudaGetErrorString(err));
+    return capture != cudaStreamCaptureStatusNone;
+}
+
 inline int div_ceil(int a, int b) {
     return (a + b - 1) / b;
 }

@@ -1011,7 +1011,8 @@ __device__ __forceinline__ void fisp_items(const FispArgs& a, const int item_beg
 // REAL (packed layouts): the real-phase excitation. Where real phases have a kernel of their own
 // (a.real_form: the real-state kernels, or this one's REAL form for sequences that those do not cover), both
 // are launched; each reads the sequence's phase flag and the one that does not match returns at once (a branch
-// that is uniform over the grid, so no host synchronisation picks the form and the pair can be captured).
+// that is uniform over the grid, so no host synchronisation picks the form and the pair can be captured). The
+// real-state kernel leaves the answer for the host, which launches only the right one as soon as it knows.
 template<int K, int G, bool PACKED = false, bool BAL = false, bool REAL = false>
 __global__ void __launch_bounds__(256, 1) fisp_epg_kernel(FispArgs a, int ntiles, int* handoff, unsigned int* status) {
     extern __shared__ float2 samples[];  // [W][32][VB]
@@ -1240,7 +1241,7 @@ FispLaunch fisp_default_launch(int N, int64_t nvoxels, int P) {
     return L;
 }
 
-const Array<float, 3>& fisp_excite_table(const CompasContext& ctx, const FISPSequence& seq) {
+FispTable fisp_excite_table(const CompasContext& ctx, const FISPSequence& seq) {
     auto& cache = *seq.cache;
     std::lock_guard<std::mutex> lock(cache.mutex);
     if (!cache.table || cache.key_rf != seq.RF_train.data() || cache.key_sp != seq.sliceprofiles.data()) {
@@ -1265,45 +1266,45 @@ const Array<float, 3>& fisp_excite_table(const CompasContext& ctx, const FISPSeq
         cache.key_rf = seq.RF_train.data();
         cache.key_sp = seq.sliceprofiles.data();
         cache.real_phases = -1;
+        cache.answer = std::make_shared<detail::HostFlag>();
     }
-    return *cache.table;
+    if (cache.real_phases < 0) cache.real_phases = cache.answer->value();
+    return FispTable {cache.table, cache.real_phases, cache.answer};
 }
 
 bool fisp_sequence_real_phases(const CompasContext& ctx, const FISPSequence& seq) {
-    const auto& tab = fisp_excite_table(ctx, seq);
-    auto& cache = *seq.cache;
-    std::lock_guard<std::mutex> lock(cache.mutex);
-    if (cache.real_phases < 0) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        COMPAS_CUDA_CHECK(cudaStreamIsCapturing(ctx.stream(), &capture));
-        if (capture != cudaStreamCaptureStatusNone) return false;  // the general form is right for every sequence
+    FispTable tab = fisp_excite_table(ctx, seq);
+    if (tab.real < 0) {
+        if (stream_captured(ctx.stream())) return false;  // the general form is right for every sequence
         const int64_t flag_at = int64_t(seq.sliceprofiles.size(0)) * seq.RF_train.size() * 4;
         float flag = 1.0f;
         DeviceGuard guard(ctx.device());
-        COMPAS_CUDA_CHECK(cudaMemcpyAsync(&flag, tab.data() + flag_at, sizeof(float), cudaMemcpyDeviceToHost,
+        COMPAS_CUDA_CHECK(cudaMemcpyAsync(&flag, tab.table->data() + flag_at, sizeof(float), cudaMemcpyDeviceToHost,
                                           ctx.stream()));
         COMPAS_CUDA_CHECK(cudaStreamSynchronize(ctx.stream()));
-        cache.real_phases = flag == 0.0f ? 1 : 0;
+        tab.real = flag == 0.0f ? 1 : 0;
+        std::lock_guard<std::mutex> lock(seq.cache->mutex);
+        if (seq.cache->table == tab.table) seq.cache->real_phases = tab.real;
     }
-    return cache.real_phases == 1;
+    return tab.real == 1;
 }
 
 kernels::FispArgs fisp_args(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
-                            const FISPSequence& seq, cfloat* echo, int64_t echo_stride) {
+                            const FISPSequence& seq, cfloat* echo, int64_t echo_stride, RealForm* form) {
     const int nTR = int(seq.RF_train.size());
     const int P = int(seq.sliceprofiles.size(0));
     const int N = seq.max_state;
     if (N < 1 || N > 128) COMPAS_ERROR("max_state must be in [1, 128]");
     COMPAS_CHECK(seq.undersampling_factor >= 1 && seq.repetitions >= 1);
     COMPAS_CHECK(P >= 1 && int(seq.sliceprofiles.size(1)) == nTR);
-    const auto& tab = fisp_excite_table(ctx, seq);
+    const FispTable tab = fisp_excite_table(ctx, seq);
 
     kernels::FispArgs a;
     a.params = params.data.data();
     a.param_stride = params.data.size(1);
     a.voxel_begin = voxel_begin;
     a.nvoxels = nvoxels;
-    a.table = reinterpret_cast<const float4*>(tab.data());
+    a.table = reinterpret_cast<const float4*>(tab.table->data());
     a.nTR = nTR;
     a.P = P;
     a.N = N;
@@ -1320,6 +1321,11 @@ kernels::FispArgs fisp_args(const CompasContext& ctx, const TissueParameters& pa
     a.dT1 = a.dT2 = nullptr;
     a.skip = nullptr;
     a.real_form = 0;
+    if (form != nullptr) {
+        form->real = tab.real;
+        if (tab.real < 0 && tab.table->stream() == ctx.stream() && !stream_captured(ctx.stream()))
+            form->ask = {tab.answer->word(), tab.answer->code()};
+    }
     return a;
 }
 
@@ -1361,7 +1367,8 @@ void launch_fisp(const CompasContext& ctx, const TissueParameters& params, int v
         return;
     }
     if (L.config < 0) L = fisp_default_launch(N, nvoxels, P);
-    kernels::FispArgs a = fisp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride);
+    RealForm form;
+    kernels::FispArgs a = fisp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride, &form);
     a.skip = skip;
     const auto& cfg = checked_config(L, N);
     const int VB = 32 / cfg.G;
@@ -1397,13 +1404,13 @@ void launch_fisp(const CompasContext& ctx, const TissueParameters& params, int v
     };
     // real phases: on the real-state kernels, else (transverse states that live through a wait) on the real-phase
     // form of a packed layout (24 operations per state against 26: 25 states, 9 positions, 9216 voxels, two
-    // repetitions of 150 TRs 616 us, 675 in the general form). Both forms are launched, the one that does not
-    // match the sequence returns at once.
+    // repetitions of 150 TRs 616 us, 675 in the general form). Until the host knows the phases both forms are
+    // launched and the one that does not match the sequence returns at once; that launch costs 2 to 4 us.
     const bool real_states = fisp_real_covers(seq, false);
     a.real_form = real_states || cfg.fn_real != nullptr;
-    if (real_states) launch_fisp_real(ctx, a, balance, handoff, handoff_capacity);
-    else if (cfg.fn_real != nullptr) run(cfg.fn_real, cfg.balanced_real);
-    run(cfg.fn, cfg.balanced);
+    if (form.real != 0 && real_states) launch_fisp_real(ctx, a, form.ask, balance, handoff, handoff_capacity);
+    else if (form.real != 0 && cfg.fn_real != nullptr) run(cfg.fn_real, cfg.balanced_real);
+    if (form.real != 1 || !a.real_form) run(cfg.fn, cfg.balanced);
 }
 
 int fisp_tangent_config_count() {
@@ -1459,7 +1466,8 @@ void launch_fisp_tangent(const CompasContext& ctx, const TissueParameters& param
     const int nTR = int(seq.RF_train.size());
     const int P = int(seq.sliceprofiles.size(0));
     const int N = seq.max_state;
-    kernels::FispArgs a = fisp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride);  // validates
+    RealForm form;
+    kernels::FispArgs a = fisp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride, &form);  // validates
     if (nvoxels <= 0 || nTR <= 0) return;
     if (L.config < 0) L = fisp_tangent_default_launch(N, nvoxels, P);
     COMPAS_CHECK(L.config >= 0 && L.config < kFispTangentConfigCount);
@@ -1483,9 +1491,9 @@ void launch_fisp_tangent(const CompasContext& ctx, const TissueParameters& param
     };
     const bool real_states = fisp_real_covers(seq, true);  // as launch_fisp
     a.real_form = real_states || fn_real != nullptr;
-    if (real_states) launch_fisp_real_tangent(ctx, a);
-    else if (fn_real != nullptr) run(fn_real);
-    run(fn);
+    if (form.real != 0 && real_states) launch_fisp_real_tangent(ctx, a, form.ask);
+    else if (form.real != 0 && fn_real != nullptr) run(fn_real);
+    if (form.real != 1 || !a.real_form) run(fn);
 }
 
 int fisp_tangent_tile_voxels(FispLaunch L) {

@@ -49,8 +49,8 @@ int fisp_real_queue_warps(int N, int P, int64_t tiles) {
     return fisp_real_warps(real_layout(N).warps, P, tiles);
 }
 
-void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& a, bool balance, int* handoff,
-                      int handoff_capacity) {
+void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& a, const kernels::HostAnswer& ask,
+                      bool balance, int* handoff, int handoff_capacity) {
     const RealLayout* layout = &real_layout(a.N);
     // Few (voxel, position) pairs leave most schedulers without a warp, and a lone warp runs at the
     // latency of its instructions: then the states go over 4 lanes.
@@ -84,7 +84,8 @@ void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& a, bool
         }
         COMPAS_CUDA_CHECK(cudaMemsetAsync(handoff, 0, sizeof(int) * size_t(grid), ctx.stream()));
     }
-    (balanced ? layout->balanced : layout->fn)<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles, handoff, ctx.status_word());
+    (balanced ? layout->balanced : layout->fn)<<<grid, 32 * W, smem, ctx.stream()>>>(a, ask, ntiles, handoff,
+                                                                                       ctx.status_word());
     check_launch("fisp_real_kernel");
 }
 

@@ -451,9 +451,10 @@ constexpr int kRealWarps = KP * PLANES <= 8 ? 16 : KP * PLANES <= 12 ? 12 : 8;
 // items, see fisp_epg_kernel.
 template<template<int, int> class State, int KP, int G, bool BAL>
 __global__ void __launch_bounds__(32 * kRealWarps<KP, State<KP, G>::kPlanes>, 1)
-    fisp_real_kernel(FispArgs a, int ntiles, int* handoff, unsigned int* status) {
+    fisp_real_kernel(FispArgs a, HostAnswer ask, int ntiles, int* handoff, unsigned int* status) {
     extern __shared__ float2 smem[];
     if (a.skip != nullptr && *a.skip != 0) return;  // uniform over the grid
+    answer_host(ask, fisp_real_phases(a));
     if (!fisp_real_phases(a)) return;
     if constexpr (BAL) {
         __shared__ FispOrder ord;
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(32 * kRealWarps<KP, State<KP, G>::kPlanes>, 1)
 // and 31.6 / 53.8; tangents of 25 states 109 / 95 and 173 / 162, of 8 states 93.5 / 56.6 and 93.6 / 104.
 constexpr int64_t kRealSplitPairs = 148 * 3 * 32;
 
-using RealKernel = void (*)(kernels::FispArgs, int, int*, unsigned int*);
+using RealKernel = void (*)(kernels::FispArgs, kernels::HostAnswer, int, int*, unsigned int*);
 using RealQueueKernel = void (*)(const kernels::FispArgs*, const int2*, int, int*);
 struct RealLayout {
     int KP, G;     // states 0 .. 2·KP·G

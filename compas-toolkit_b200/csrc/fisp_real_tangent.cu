@@ -44,7 +44,7 @@ int fisp_real_tangent_tile_voxels(int N) {
     return 32 / real_layout(N).G;
 }
 
-void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& a) {
+void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& a, const kernels::HostAnswer& ask) {
     const RealLayout* layout = &real_layout(a.N);
     if (int64_t(a.nvoxels) * a.P <= kRealSplitPairs) layout = &covering(kSplitLayouts, 4, a.N);
     const int ntiles = div_ceil(a.nvoxels, 32 / layout->G);
@@ -54,7 +54,7 @@ void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs&
     const void* fn = reinterpret_cast<const void*>(layout->fn);
     allow_smem(fn, smem);
     const int grid = std::min(ntiles, resident_ctas(fn, 32 * W, smem, ctx.device()));
-    layout->fn<<<grid, 32 * W, smem, ctx.stream()>>>(a, ntiles, nullptr, nullptr);
+    layout->fn<<<grid, 32 * W, smem, ctx.stream()>>>(a, ask, ntiles, nullptr, nullptr);
     check_launch("fisp_real_kernel (tangents)");
 }
 

@@ -19,7 +19,12 @@ bool fisp_config_info(int index, int* K, int* G);
 bool fisp_config_packed(int index);  // EPGPacked layout (two states per FFMA2)
 FispLaunch fisp_default_launch(int N, int64_t nvoxels, int P);
 FispLaunch tuned_fisp_launch(int N, int64_t nvoxels, int P);
-const Array<float, 3>& fisp_excite_table(const CompasContext& ctx, const FISPSequence& seq);
+struct FispTable {
+    std::shared_ptr<Array<float, 3>> table;
+    int real;  // every phase real: 1, 0, or -1 when the host does not know it yet
+    std::shared_ptr<detail::HostFlag> answer;
+};
+FispTable fisp_excite_table(const CompasContext& ctx, const FISPSequence& seq);
 // whether every RF and slice-profile phase of the sequence is real (sin φ = 0), read back from its
 // excitation table: synchronises the context's stream the first time (not while it is captured)
 bool fisp_sequence_real_phases(const CompasContext& ctx, const FISPSequence& seq);
@@ -34,9 +39,16 @@ bool fisp_sequence_real_phases(const CompasContext& ctx, const FISPSequence& seq
 void launch_fisp(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
                  const FISPSequence& seq, cfloat* echo, int64_t echo_stride, FispLaunch L,
                  const int* skip = nullptr, bool balance = false, int* handoff = nullptr, int handoff_capacity = 0);
+// Whether a sequence's phases (RF) are real, as far as the host knows: 1, 0, or -1 with the question to pass to the
+// real-state (real-RF) kernel (on the stream that built the table, so that the answer is of the finished table, and
+// not while it is captured: a replay would give it long after).
+struct RealForm {
+    int real = -1;
+    kernels::HostAnswer ask;
+};
 // argument block of one FISP simulation (validates the sequence, builds its table on first use)
 kernels::FispArgs fisp_args(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
-                            const FISPSequence& seq, cfloat* echo, int64_t echo_stride);
+                            const FISPSequence& seq, cfloat* echo, int64_t echo_stride, RealForm* form = nullptr);
 int fisp_tile_voxels(FispLaunch L);  // voxels per work item (tile) of layout L
 // persistent work-queue launch over (job, tile) items of FISP jobs that all use layout L;
 // *head must be 0 when the kernel starts. `real`: every job's phases are real
@@ -50,9 +62,9 @@ void launch_fisp_queue(cudaStream_t stream, int device, FispLaunch L, int max_st
 bool fisp_real_covers(const FISPSequence& seq, bool tangents);
 int fisp_real_warps(int most, int P, int64_t tiles);  // warps per CTA for runs of `tiles` tiles
 bool fisp_layout_forced(int N, bool tangents);        // an explicit override names a general layout that holds N states
-void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& args, bool balance, int* handoff,
-                      int handoff_capacity);
-void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& args);
+void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& args, const kernels::HostAnswer& ask,
+                      bool balance, int* handoff, int handoff_capacity);
+void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& args, const kernels::HostAnswer& ask);
 // work queues: items of tiles of 32 voxels (tangents: fisp_real_tangent_tile_voxels), W warps per CTA
 int fisp_real_queue_warps(int N, int P, int64_t tiles);
 int fisp_real_tangent_queue_warps(int N, int P, int64_t tiles);
@@ -94,7 +106,8 @@ void launch_pssfp(const CompasContext& ctx, const TissueParameters& params, int 
                   const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride, PssfpLaunch L,
                   const int* skip = nullptr);
 kernels::PssfpArgs pssfp_args(const CompasContext& ctx, const TissueParameters& params, int voxel_begin,
-                              int nvoxels, const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride);
+                              int nvoxels, const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride,
+                              RealForm* form = nullptr);
 int pssfp_tile_voxels(PssfpLaunch L);
 // value and T1/T2 tangents (forward mode) in one launch of layout L
 void launch_pssfp_tangent(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,

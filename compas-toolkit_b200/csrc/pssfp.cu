@@ -535,7 +535,8 @@ __device__ __forceinline__ void pssfp_tile_packed(const PssfpArgs& a, const int 
 
 // PACKED: ZT/2 pairs of isochromats per lane in the two-wide layout (pssfp_tile_packed). Sequences with
 // real RF run on the kernels of pssfp_real.cuh, launched beside these: each reads the table's flag and
-// the one that does not match returns at once (uniform over the grid).
+// the one that does not match returns at once (uniform over the grid). The real-RF kernel leaves the answer for
+// the host, which launches only the right one as soon as it knows.
 template<int ZT, int GZ, bool PACKED = false>
 __global__ void __launch_bounds__(128) pssfp_kernel(PssfpArgs a) {
     if (a.skip != nullptr && *a.skip != 0) return;  // uniform over the grid
@@ -680,7 +681,7 @@ PssfpLaunch pssfp_real_default_launch(int nz, int64_t nvoxels) {
 }
 
 kernels::PssfpArgs pssfp_args(const CompasContext& ctx, const TissueParameters& params, int voxel_begin,
-                              int nvoxels, const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride) {
+                              int nvoxels, const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride, RealForm* form) {
     const int nTR = int(seq.RF_train.size());
     const int nRF = int(seq.gamma_dt_RF.size());
     const int nz = int(seq.z.size());
@@ -688,6 +689,8 @@ kernels::PssfpArgs pssfp_args(const CompasContext& ctx, const TissueParameters& 
     if (nz > 64) COMPAS_ERROR("pSSFP supports at most 64 z positions");
     DeviceGuard guard(ctx.device());
     std::shared_ptr<Array<cfloat, 2>> zap;
+    std::shared_ptr<detail::HostFlag> answer;
+    int known = -1;
     {
         auto& cache = *seq.cache;
         std::lock_guard<std::mutex> lock(cache.mutex);
@@ -709,8 +712,12 @@ kernels::PssfpArgs pssfp_args(const CompasContext& ctx, const TissueParameters& 
             cache.key_rf = seq.RF_train.data();
             cache.key_g = seq.gamma_dt_RF.data();
             cache.real_rf = -1;
+            cache.answer = std::make_shared<detail::HostFlag>();
         }
+        if (cache.real_rf < 0) cache.real_rf = cache.answer->value();
         zap = cache.table;
+        answer = cache.answer;
+        known = cache.real_rf;
     }
     kernels::PssfpArgs a;
     a.params = params.data.data();
@@ -731,6 +738,11 @@ kernels::PssfpArgs pssfp_args(const CompasContext& ctx, const TissueParameters& 
     a.echo_stride = echo_stride;
     a.dT1 = a.dT2 = nullptr;
     a.skip = nullptr;
+    if (form != nullptr) {
+        form->real = known;
+        if (known < 0 && zap->stream() == ctx.stream() && !stream_captured(ctx.stream()))
+            form->ask = {answer->word(), answer->code()};
+    }
     return a;
 }
 
@@ -755,18 +767,22 @@ int pssfp_tile_voxels(PssfpLaunch L) {
 void launch_pssfp(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
                   const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride, PssfpLaunch L, const int* skip) {
     const int nz = int(seq.z.size());
-    kernels::PssfpArgs a = pssfp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride);
+    RealForm form;
+    kernels::PssfpArgs a = pssfp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride, &form);
     a.skip = skip;
     if (nvoxels <= 0) return;
     if (L.config < 0) L = pssfp_default_launch(nz, nvoxels);
     const auto& cfg = checked_config(L, nz);
     DeviceGuard guard(ctx.device());
-    const unsigned grid = pssfp_grid(nvoxels, cfg.GZ);
-    cfg.fn<<<grid, kPssfpThreads, 0, ctx.stream()>>>(a);
-    check_launch("pssfp_kernel");
-    // the form that does not match the sequence returns at once
+    // until the host knows which, both forms are launched, and the one that does not match the sequence
+    // returns at once
+    if (form.real != 1) {
+        cfg.fn<<<pssfp_grid(nvoxels, cfg.GZ), kPssfpThreads, 0, ctx.stream()>>>(a);
+        check_launch("pssfp_kernel");
+    }
+    if (form.real == 0) return;
     const auto& real = checked_config(tuned_pssfp_launch(nz, nvoxels, true), nz);
-    pssfp_real_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a);
+    pssfp_real_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a, form.ask);
     check_launch("pssfp_real_kernel");
 }
 
@@ -800,21 +816,22 @@ void launch_pssfp_tangent_queue(cudaStream_t stream, int device, PssfpLaunch L, 
 }
 
 bool pssfp_sequence_real_rf(const CompasContext& ctx, const pSSFPSequence& seq) {
-    kernels::PssfpArgs a = pssfp_args(ctx, TissueParameters {}, 0, 0, seq, nullptr, 0);  // builds the table
-    auto& cache = *seq.cache;
-    std::lock_guard<std::mutex> lock(cache.mutex);
-    if (cache.real_rf < 0) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        COMPAS_CUDA_CHECK(cudaStreamIsCapturing(ctx.stream(), &capture));
-        if (capture != cudaStreamCaptureStatusNone) return false;  // the general form is right for every sequence
+    RealForm form;
+    const kernels::PssfpArgs a = pssfp_args(ctx, TissueParameters {}, 0, 0, seq, nullptr, 0, &form);  // builds the table
+    int real = form.real;
+    if (real < 0) {
+        if (stream_captured(ctx.stream())) return false;  // the general form is right for every sequence
         float2 flag = make_float2(1.0f, 0.0f);
         DeviceGuard guard(ctx.device());
         COMPAS_CUDA_CHECK(cudaMemcpyAsync(&flag, a.zap + int64_t(a.nTR + 1) * a.nRF, sizeof(float2),
                                           cudaMemcpyDeviceToHost, ctx.stream()));
         COMPAS_CUDA_CHECK(cudaStreamSynchronize(ctx.stream()));
-        cache.real_rf = flag.x == 0.0f ? 1 : 0;
+        real = flag.x == 0.0f ? 1 : 0;
+        auto& cache = *seq.cache;
+        std::lock_guard<std::mutex> lock(cache.mutex);
+        if (cache.table && reinterpret_cast<const float2*>(cache.table->data()) == a.zap) cache.real_rf = real;
     }
-    return cache.real_rf == 1;
+    return real == 1;
 }
 
 // Value and T1/T2 tangents in one launch, with the value kernel's layout L.
@@ -822,18 +839,21 @@ void launch_pssfp_tangent(const CompasContext& ctx, const TissueParameters& para
                           const pSSFPSequence& seq, cfloat* echo, cfloat* dT1, cfloat* dT2, int64_t echo_stride,
                           PssfpLaunch L) {
     const int nz = int(seq.z.size());
-    kernels::PssfpArgs a = pssfp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride);
+    RealForm form;
+    kernels::PssfpArgs a = pssfp_args(ctx, params, voxel_begin, nvoxels, seq, echo, echo_stride, &form);
     if (nvoxels <= 0) return;
     if (L.config < 0) L = pssfp_default_launch(nz, nvoxels);
     const auto& cfg = checked_config(L, nz);
     a.dT1 = reinterpret_cast<float2*>(dT1);
     a.dT2 = reinterpret_cast<float2*>(dT2);
     DeviceGuard guard(ctx.device());
-    const unsigned grid = pssfp_grid(nvoxels, cfg.GZ);
-    cfg.tangent<<<grid, kPssfpThreads, 0, ctx.stream()>>>(a);
-    check_launch("pssfp_tangent_kernel");
+    if (form.real != 1) {
+        cfg.tangent<<<pssfp_grid(nvoxels, cfg.GZ), kPssfpThreads, 0, ctx.stream()>>>(a);
+        check_launch("pssfp_tangent_kernel");
+    }
+    if (form.real == 0) return;
     const auto& real = checked_config(tuned_pssfp_launch(nz, nvoxels, true), nz);
-    pssfp_real_tangent_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a);
+    pssfp_real_tangent_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a, form.ask);
     check_launch("pssfp_real_kernel (tangents)");
 }
 

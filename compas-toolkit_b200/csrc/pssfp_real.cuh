@@ -395,8 +395,9 @@ __device__ __forceinline__ bool pssfp_real_rf(const PssfpArgs& a) {
 // One simulation (TAN: with its T1 and T2 tangents into a.dT1, a.dT2). Returns at once when the RF is not
 // real: the general kernel launched beside it runs then.
 template<int ZT, int GZ, bool TAN>
-__global__ void __launch_bounds__(128) pssfp_real_kernel(PssfpArgs a) {
+__global__ void __launch_bounds__(128) pssfp_real_kernel(PssfpArgs a, HostAnswer ask) {
     if (!TAN && a.skip != nullptr && *a.skip != 0) return;  // uniform over the grid
+    answer_host(ask, pssfp_real_rf(a));
     if (!pssfp_real_rf(a)) return;
     pssfp_real_tile<ZT, GZ, TAN>(a, blockIdx.x);
 }
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(128) pssfp_real_queue_kernel(const PssfpArgs* 
 
 struct PssfpRealKernels {
     int ZT, GZ;
-    void (*fn)(kernels::PssfpArgs);
+    void (*fn)(kernels::PssfpArgs, kernels::HostAnswer);
     void (*queue)(const kernels::PssfpArgs*, const int2*, int, int*);
 };
 // the real-RF value and tangent kernels of a layout (every layout of pssfp.cu has them)

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <mutex>
 #include <sstream>
+#include <vector>
 
 #include "common.cuh"
 #include "compas/compas.h"
@@ -35,6 +36,25 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
 DeviceState g_devices[kMaxDevices];
 
+// The words of detail::HostFlag: one block for the process, made with the first context and kept to its end
+// (a kernel may still write to a word whose flag is gone). A sequence beyond their number runs
+// without one: its calls launch both forms.
+constexpr int kHostFlags = 1024;
+std::mutex g_flag_mutex;
+unsigned int* g_flag_words = nullptr;
+std::vector<unsigned int*> g_flag_free;
+unsigned int g_flag_ticket = 0;
+
+void make_host_flags() {
+    std::lock_guard<std::mutex> lock(g_flag_mutex);
+    if (g_flag_words != nullptr) return;
+    void* p = nullptr;
+    COMPAS_CUDA_CHECK(cudaHostAlloc(&p, kHostFlags * sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped));
+    g_flag_words = static_cast<unsigned int*>(p);
+    g_flag_free.reserve(kHostFlags);
+    for (int i = kHostFlags - 1; i >= 0; i--) g_flag_free.push_back(g_flag_words + i);
+}
+
 DeviceState& device_state(int device) {
     if (device < 0 || device >= kMaxDevices) COMPAS_ERROR("invalid device index");
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -54,6 +74,7 @@ DeviceState& device_state(int device) {
         COMPAS_CUDA_CHECK(cudaStreamCreateWithFlags(&st.stream, cudaStreamNonBlocking));
         COMPAS_CUDA_CHECK(cudaMalloc(&st.status, sizeof(unsigned int)));
         COMPAS_CUDA_CHECK(cudaMemset(st.status, 0, sizeof(unsigned int)));
+        make_host_flags();
         COMPAS_CUDA_CHECK(cudaSetDevice(prev));
         st.ready = true;
     }
@@ -84,6 +105,31 @@ cudaStream_t device_stream(int device) {
 
 unsigned int* device_status_word(int device) {
     return device_state(device).status;
+}
+
+HostFlag::HostFlag() : m_word(nullptr), m_ticket(0) {
+    std::lock_guard<std::mutex> lock(g_flag_mutex);
+    if (g_flag_free.empty()) return;
+    m_word = g_flag_free.back();
+    g_flag_free.pop_back();
+    // 31 bits, never 0: what a word holds from its earlier users, or gets from their kernels still, is
+    // another ticket's and reads as unknown
+    g_flag_ticket = (g_flag_ticket + 1) & 0x7fffffffu;
+    if (g_flag_ticket == 0) g_flag_ticket = 1;
+    m_ticket = g_flag_ticket;
+    *static_cast<volatile unsigned int*>(m_word) = 0;
+}
+
+HostFlag::~HostFlag() {
+    if (m_word == nullptr) return;
+    std::lock_guard<std::mutex> lock(g_flag_mutex);
+    g_flag_free.push_back(m_word);
+}
+
+int HostFlag::value() const {
+    if (m_word == nullptr) return -1;
+    const unsigned int v = *static_cast<const volatile unsigned int*>(m_word);
+    return v >> 1 == m_ticket ? int(v & 1u) : -1;
 }
 
 Buffer::Buffer(size_t nbytes, int dev, cudaStream_t s) : bytes(nbytes), device(dev), stream(s) {

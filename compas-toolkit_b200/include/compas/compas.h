@@ -85,6 +85,23 @@ struct Buffer {
 };
 int current_device();
 cudaStream_t device_stream(int device);
+
+// One word of pinned host memory in which a kernel leaves a yes or no about a sequence's table, so that
+// later calls know it without a synchronisation.
+class HostFlag {
+  public:
+    HostFlag();
+    ~HostFlag();
+    HostFlag(const HostFlag&) = delete;
+    HostFlag& operator=(const HostFlag&) = delete;
+    unsigned int* word() const { return m_word; }  // null: no word was free, the answer stays unknown
+    unsigned int code() const { return m_ticket << 1; }  // a kernel writes code() | answer
+    int value() const;  // 0 or 1, or -1 while no answer has arrived
+
+  private:
+    unsigned int* m_word;
+    unsigned int m_ticket;  // tells this flag's answers from those of the word's earlier users
+};
 }  // namespace detail
 
 template<typename T, size_t N = 1>
@@ -301,7 +318,8 @@ struct FISPSequence: public Object {
         const void* key_rf = nullptr;
         const void* key_sp = nullptr;
         std::shared_ptr<Array<float, 3>> table;
-        int real_phases = -1;  // host copy of the table's phase flag: -1 not read yet, else 0 / 1
+        int real_phases = -1;  // host copy of the table's phase flag: -1 not known yet, else 0 / 1
+        std::shared_ptr<detail::HostFlag> answer;  // where the simulation kernels leave it
     };
     std::shared_ptr<Cache> cache = std::make_shared<Cache>();
 };
@@ -343,7 +361,8 @@ struct pSSFPSequence: public Object {
         const void* key_rf = nullptr;
         const void* key_g = nullptr;
         std::shared_ptr<Array<cfloat, 2>> table;
-        int real_rf = -1;  // host copy of the table's flag: -1 not read yet, 1 every RF sample real, else 0
+        int real_rf = -1;  // host copy of the table's flag: -1 not known yet, 1 every RF sample real, else 0
+        std::shared_ptr<detail::HostFlag> answer;  // where the simulation kernels leave it
     };
     std::shared_ptr<Cache> cache = std::make_shared<Cache>();
 };

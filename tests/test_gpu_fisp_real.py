@@ -171,3 +171,49 @@ def test_a_voxel_without_relaxation_times_stays_alone(cb, ctx):
     assert np.isfinite(got).all()
     keep = np.arange(40) != 7
     assert np.array_equal(got[:, keep], ref[:, keep])
+
+
+# ------------------------------------------------------------------------------------------------
+# one launch per simulation once the host knows a sequence's form (csrc/runtime.cu, HostFlag)
+# ------------------------------------------------------------------------------------------------
+
+def _sequence(cb, ctx, kind, turned):
+    turn = np.exp(0.4j) if turned else 1.0
+    if kind == "fisp":
+        seq = W.fisp_sequence(np.linspace(5, 60, 9) * turn, np.ones((1, 9)), 8.7e-3, 4.35e-3, 25e-3, 6)
+        return cb.FispSequence.from_dict(ctx, seq)
+    seq = W.pssfp_sequence(np.random.default_rng(3), 9, nrf=3, nz=2)
+    seq["rf"] = (seq["rf"] * turn).astype(np.complex64)
+    return cb.pSSFPSequence.from_dict(ctx, seq)
+
+
+@pytest.mark.parametrize("kind", ["fisp", "pssfp"])
+@pytest.mark.parametrize("turned", [False, True])
+@pytest.mark.parametrize("tangents", [False, True])
+def test_one_launch_once_the_form_is_known(cb, ctx, kind, turned, tangents):
+    params = cb.TissueParameters.from_soa(ctx, W.tissue_voxels(np.random.default_rng(2), 70, 22.4))
+    s = _sequence(cb, ctx, kind, turned)
+
+    def run():
+        if not tangents:
+            return cb.simulate_magnetization(ctx, params, s).to_numpy()
+        return np.stack([a.to_numpy() for a in cb.simulate_magnetization_tangents(ctx, params, s).values()])
+
+    first = run()
+    before = cb.launch_count()
+    again = run()
+    assert cb.launch_count() - before == 1
+    assert np.array_equal(first, again)
+
+
+def test_more_sequences_than_flags_and_reused_flags(cb, ctx):
+    # 1100 sequences at a time of both forms in turn, then as many others on the words they gave back
+    params = cb.TissueParameters.from_soa(ctx, W.tissue_voxels(np.random.default_rng(2), 33, 22.4))
+    ref = [cb.simulate_magnetization(ctx, params, _sequence(cb, ctx, "fisp", t)).to_numpy() for t in (False, True)]
+    for shift in (0, 1):
+        kept = [_sequence(cb, ctx, "fisp", (i + shift) % 2 == 1) for i in range(1100)]
+        for _ in range(2):
+            got = [cb.simulate_magnetization(ctx, params, s) for s in kept]
+            for i, g in enumerate(got):
+                assert np.array_equal(g.to_numpy(), ref[(i + shift) % 2]), i
+        del kept, got
