@@ -62,6 +62,12 @@ struct PssfpArgs {
     const int* skip;  // one-simulation kernel: returns at once when *skip != 0 (null: never)
 };
 
+// The order in which the real-RF pSSFP kernels sum a voxel's isochromats: groups of `group`, `lanes` (a power of
+// two) of them (pssfp_real_tile)
+struct PssfpSplit {
+    int group, lanes;
+};
+
 // Where a one-simulation kernel of real phases or real RF tells the host whether the sequence is (a
 // detail::HostFlag; word null: not asked). A parameter of its own, for those kernels alone: in the argument
 // blocks above it changed the registers of the general tangent kernels (up to 5 % slower).

@@ -93,6 +93,8 @@ void launch_fisp_tangent_queue(cudaStream_t stream, int device, FispLaunch L, in
 // ---- pSSFP ------------------------------------------------------------------------------
 struct PssfpLaunch {
     int config;  // index into the instantiated (ZT, GZ) layouts, -1 = default
+    // real-RF kernels: the order of the sum over the isochromats (kernels::PssfpSplit); 0: the layout's own
+    int group = 0, lanes = 0;
 };
 int pssfp_config_count();
 bool pssfp_config_info(int index, int* ZT, int* GZ);
@@ -100,7 +102,8 @@ bool pssfp_config_packed(int index);  // two-wide layout: ZT/2 pairs of isochrom
 PssfpLaunch pssfp_default_launch(int nz, int64_t nvoxels);
 PssfpLaunch pssfp_real_default_launch(int nz, int64_t nvoxels);
 // real: the layout of the real-RF kernels (pssfp_real.cuh), which differ from the general ones' only in
-// the default
+// the default. All defaults for one nz sum the isochromats in one order, so the echoes do not depend on nvoxels;
+// an explicit override sums in its own.
 PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels, bool real = false);
 void launch_pssfp(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
                   const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride, PssfpLaunch L,

@@ -12,12 +12,12 @@
 // that follows it. That is 12 or 14 operations per isochromat and RF sample (K and H to second or third
 // order in θ²), 24 before. Pairs of isochromats run as two-wide FP32 instructions.
 //
-// Which order, and whether the division is safe, is decided once: the order by each lane from the largest
-// axis of the sequence (the table's second flag) and its isochromats, the division by the voxel's
-// relaxation. Angles above half a radian take longer series sample by sample (and sincos above 3π/2), and a
+// Which order, and whether the division is safe, is decided once per voxel: the order from the largest
+// axis of the sequence (the table's second flag) and its isochromats, the division from its
+// relaxation. Samples whose angles may pass half a radian take longer series (and sincos above 3π/2), and a
 // voxel that a pulse outlasts by far relaxes explicitly after every sample. The warp's vote only picks the
-// cheapest of three loops that does what all its lanes need; in each of them a lane gets the same bits
-// (what it does not need enters as a factor of 1 or a highest coefficient of 0), so a voxel's echoes
+// cheapest of three loops that does what all its voxels need; in each of them a voxel gets the same bits
+// (what it does not need enters as a factor of 1 or a highest coefficient of 0), so its echoes
 // do not depend on its neighbours. Loop 2, in us for 20000 voxels, 60 TRs of 15 samples, 9 / 35 z (with the
 // 24-operation rotation in brackets): 30 % of the voxels with T2 = 0 338 / 662 (350 / 729; no such voxel, loop
 // 0: 170 / 394), az of 1 rad at the outer z 549 / 1523 (1349 / 2810); pulses of one sample of 40° 61 / 125 (139 / 219).
@@ -52,33 +52,32 @@ __device__ __forceinline__ T vset(float s) {
 struct RealSample {
     float nb0, nb1, nb2;  // -B·E2^-i, -B·(E1/E2)^i, -B·(E2/E1)^i, B = ±ax
     float nax2;           // -ax²
+    bool small;           // θ² ≤ 1/4 for every isochromat of the voxel
 };
 
-// What a lane needs of the loop it runs in (file header)
+// What a voxel needs of the loop it runs in (file header)
 struct RealNeeds {
     float k6, h6;   // highest coefficients of K and -H: those of the third order, or 0
-    float y_min;    // no short series below this -θ²: -1/4, or -inf when no sample has more
     float E1, E2;   // the relaxation after a sample where it is not divided out, else 1
 };
 
-// sin θ/θ, (1 - cos θ)/θ², cos θ for y = -θ²
+// -sin θ/θ, -(1 - cos θ)/θ², -cos θ for y = -θ² of a large angle, or NaN
 struct RealRotation {
-    float s, h, c;
+    float ns, nh, nc;
 };
-static __device__ __noinline__ RealRotation real_rotation(float y) {  // rarely run: one copy of the sincos
+static __device__ __noinline__ RealRotation real_sincos(float y) {  // rarely run: one copy of the sincos
     RealRotation q;
-    if (y >= -0.25f) {  // Taylor, the next terms are below 1e-8
-        q.s = fmaf(y, fmaf(y, fmaf(y, 1.0f / 5040.0f, 1.0f / 120.0f), 1.0f / 6.0f), 1.0f);
-        q.h = fmaf(y, fmaf(y, fmaf(y, 1.0f / 40320.0f, 1.0f / 720.0f), 1.0f / 24.0f), 0.5f);
-        q.c = fmaf(y, q.h, 1.0f);
-    } else {
-        const float t2 = -y, th = sqrtf(t2);
-        float sn;
-        sincosf(th, &sn, &q.c);
-        q.s = sn / th;
-        q.h = (1.0f - q.c) / t2;
-    }
+    const float th = sqrtf(-y);
+    float sn, cs;
+    sincosf(th, &sn, &cs);
+    q.ns = -sn / th;
+    q.nh = (1.0f - cs) / y;
+    q.nc = -cs;
     return q;
+}
+__device__ __forceinline__ void real_rotation(float y, float& ns, float& nh, float& nc) {
+    const RealRotation q = real_sincos(y);
+    ns = q.ns, nh = q.nh, nc = q.nc;
 }
 
 // -sin θ/θ, -(1 - cos θ)/θ², -cos θ for y = -θ² ≥ kRealSeriesMin (θ ≤ 3π/2) on an isochromat or a pair, from
@@ -118,12 +117,7 @@ __device__ __forceinline__ void real_step(T (&v)[TAN ? 9 : 3], T A, T nA, const 
                                           float t1, float t2) {
     const T y = vfma(nA, A, vset<T>(f.nax2));  // -θ²
     const T nb0 = vset<T>(f.nb0), nb1 = vset<T>(f.nb1), nb2 = vset<T>(f.nb2);
-    bool taylor = true;
-    if constexpr (LOOP == 2) {
-        if constexpr (sizeof(T) == 4) taylor = y >= need.y_min;
-        else taylor = y.x >= need.y_min && y.y >= need.y_min;
-    }
-    if (taylor) {
+    if (LOOP < 2 || f.small) {
         T K, nH;
         if constexpr (LOOP == 0) {
             K = vfma(y, vfma(y, vset<T>(-1.0f / 360.0f), vset<T>(1.0f / 6.0f)), vset<T>(2.0f));
@@ -144,20 +138,12 @@ __device__ __forceinline__ void real_step(T (&v)[TAN ? 9 : 3], T A, T nA, const 
         }
     } else {
         T nS, nH, c;
+        real_series(y, nS, nH, c);
         if constexpr (sizeof(T) == 4) {
-            if (y >= kRealSeriesMin) {
-                real_series(y, nS, nH, c);
-            } else {
-                const RealRotation r = real_rotation(y);
-                nS = -r.s, nH = -r.h, c = -r.c;
-            }
-        } else {
-            if (y.x >= kRealSeriesMin && y.y >= kRealSeriesMin) {
-                real_series(y, nS, nH, c);
-            } else {
-                const RealRotation r0 = real_rotation(y.x), r1 = real_rotation(y.y);
-                nS = make_float2(-r0.s, -r1.s), nH = make_float2(-r0.h, -r1.h), c = make_float2(-r0.c, -r1.c);
-            }
+            if (!(y >= kRealSeriesMin)) real_rotation(y, nS, nH, c);
+        } else if (!(y.x >= kRealSeriesMin && y.y >= kRealSeriesMin)) {
+            if (!(y.x >= kRealSeriesMin)) real_rotation(y.x, nS.x, nH.x, c.x);
+            if (!(y.y >= kRealSeriesMin)) real_rotation(y.y, nS.y, nH.y, c.y);
         }
 #pragma unroll
         for (int q = 0; q < (TAN ? 3 : 1); q++) {
@@ -204,13 +190,24 @@ __device__ __forceinline__ void real_precess(T (&v)[TAN ? 9 : 3], T c, T sn, T n
     }
 }
 
-// One tile (128/GZ voxels) of a simulation: GZ lanes per voxel, ZT isochromats per lane, slots p and
+// One tile (128/GZ voxels) of a simulation: GZ lanes per voxel, up to ZT isochromats per lane, slots p and
 // p + ZT/2 in a pair, an odd last slot by itself.
+//
+// The echo is the sum over the isochromats in an order that belongs to their number alone: one after the
+// other within the groups of split.group, and those as a tree over the split.lanes groups. That is the
+// order of the layout of many voxels, a group to a lane. A layout of more lanes deals a group out to `parts`
+// neighbouring lanes in chunks of ZT and passes the running sum along them. What a lane needs follows from all the
+// isochromats of its voxel, so the echoes are the same bits in every layout: one simulation takes the
+// layout for its voxels, a batch the one for all its voxels.
 template<int ZT, int GZ, bool TAN>
-__device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int tile) {
+__device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const PssfpSplit split, const int tile) {
     constexpr int ZP = ZT / 2, ODD = ZT % 2, ZA = ZP > 0 ? ZP : 1, NV = TAN ? 9 : 3;
     const int lane = threadIdx.x & 31;
     const int sub = lane % GZ;
+    const int parts = GZ == 1 ? 1 : (split.group + ZT - 1) / ZT;
+    const int group = GZ == 1 ? 0 : sub / parts, part = GZ == 1 ? 0 : sub % parts;
+    const int first = group * split.group + part * ZT;  // the lane's first isochromat
+    const int count = min(min(ZT, split.group - part * ZT), a.nz - first);  // and their number (or none, ≤ 0)
     const int vloc = (tile * blockDim.x + threadIdx.x) / GZ;
     const bool vok = vloc < a.nvoxels;
     const int64_t vcol = a.voxel_begin + (vok ? vloc : a.nvoxels - 1);
@@ -232,20 +229,17 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
     // inversion: mz = cos(πB1), then relaxation (isochromat.cuh:100-112); z - 1 and its T1 derivative
     const float z0 = __fmul_rn(E1_inv, __fadd_rn(cospif(B1), -1.0f));
     const float z0_1 = a.dt_inv * R1 * R1 * z0;
-    auto position = [&](int k) {
-        const int zi = sub * ZT + k;
-        return zi < a.nz ? a.z[zi] : 0.0f;
-    };
-    auto axis = [&](float z) {
+    auto position = [&](int k) { return k < count ? a.z[first + k] : 0.0f; };
+    auto axis = [&](int k, float z) {
         const float v = __fmaf_rn(-a.gz_ex, z, -(a.dt_ex * kTwoPi * B0));
-        azmax2 = fmaxf(azmax2, v * v);
+        if (k < count) azmax2 = fmaxf(azmax2, v * v);
         return v;
     };
     auto angle = [&](float g, float z) { return __fmaf_rn(-(g * a.gz_pr), z, -(a.dt_pr * kTwoPi * B0)); };
 #pragma unroll
     for (int p = 0; p < ZP; p++) {
         const float zl = position(p), zh = position(p + ZP);
-        az[p] = make_float2(axis(zl), axis(zh));
+        az[p] = make_float2(axis(p, zl), axis(p + ZP, zh));
         naz[p] = make_float2(-az[p].x, -az[p].y);
         sincosf(angle(1.0f, zl), &spr[p].x, &cpr[p].x);
         sincosf(angle(1.0f, zh), &spr[p].y, &cpr[p].y);
@@ -255,14 +249,16 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
     }
     if constexpr (ODD) {
         const float z = position(2 * ZP);
-        oaz = axis(z);
+        oaz = axis(2 * ZP, z);
         sincosf(angle(1.0f, z), &ospr, &ocpr);
 #pragma unroll
         for (int q = 0; q < NV; q++) O[q] = q == 2 ? z0 : q == 5 ? z0_1 : 0.f;
     }
 
-    // what the lane needs: its largest angle of any sample, and whether the voxel's E1 and E2 to the power of
+    // what the voxel needs: its largest angle of any sample, and whether its E1 and E2 to the power of
     // the pulse's samples stay far from the ends of the range (a NaN fails every comparison)
+#pragma unroll
+    for (int d = GZ / 2; d > 0; d /= 2) azmax2 = fmaxf(azmax2, __shfl_xor_sync(0xffffffffu, azmax2, d, GZ));
     const float zap_max = __ldg(&a.zap[int64_t(a.nTR + 1) * a.nRF].y);
     const float th2 = __fmaf_rn(zap_max * B1, zap_max * B1, azmax2);
     const float pulse = float(a.nRF) * a.dt_ex * fmaxf(fabsf(R1), fabsf(R2));
@@ -270,7 +266,6 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
     RealNeeds need;
     need.k6 = second ? 0.0f : 1.0f / 15120.0f;
     need.h6 = second ? 0.0f : -1.0f / 40320.0f;
-    need.y_min = third ? -INFINITY : -0.25f;
     need.E1 = scaled ? 1.0f : E1_ex;
     need.E2 = scaled ? 1.0f : E2_ex;
     const int loop = !__all_sync(0xffffffffu, scaled && third) ? 2 : __all_sync(0xffffffffu, second) ? 0 : 1;
@@ -296,6 +291,7 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
             f.nb1 = __fmul_rn(nb, f1);
             f.nb2 = __fmul_rn(nb, f2);
             f.nax2 = -__fmul_rn(ax, ax);
+            f.small = LOOP < 2 || __fmaf_rn(ax, ax, azmax2) <= 0.25f;
             f0 = __fmaf_rn(f0, g0, f0);
             f1 = __fmaf_rn(f1, g1, f1);
             f2 = __fmaf_rn(f2, g2, f2);
@@ -351,32 +347,76 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int ti
             pulse_of(t + 1);
             precess(E1_first, E2_first);
             const int64_t at = int64_t(t) * a.echo_stride + a.voxel_begin + vloc;
-#pragma unroll
-            for (int q = 0; q < NV; q += 3) {
-                float sx = 0.0f, sy = 0.0f;  // over the slots in order
+            constexpr int NQ = NV / 3;
+            float sx[NQ], sy[NQ];
+            auto add_slots = [&](int n, float& x, float& y) __attribute__((always_inline)) {  // in order
+                const int q = 3 * n;
 #pragma unroll
                 for (int p = 0; p < ZP; p++)
-                    if (sub * ZT + p < a.nz) {
-                        sx += P[p][q].x;
-                        sy += P[p][q + 1].x;
+                    if (p < count) {
+                        x += P[p][q].x;
+                        y += P[p][q + 1].x;
                     }
 #pragma unroll
                 for (int p = 0; p < ZP; p++)
-                    if (sub * ZT + p + ZP < a.nz) {
-                        sx += P[p][q].y;
-                        sy += P[p][q + 1].y;
+                    if (p + ZP < count) {
+                        x += P[p][q].y;
+                        y += P[p][q + 1].y;
                     }
-                if (ODD && sub * ZT + 2 * ZP < a.nz) {
-                    sx += O[q];
-                    sy += O[q + 1];
+                if (ODD && 2 * ZP < count) {
+                    x += O[q];
+                    y += O[q + 1];
                 }
+            };
+#pragma unroll
+            for (int n = 0; n < NQ; n++) {
+                sx[n] = sy[n] = 0.0f;
+                add_slots(n, sx[n], sy[n]);
+            }
+            if (GZ == 1 || parts == 1) {
 #pragma unroll
                 for (int d = GZ / 2; d > 0; d /= 2) {
-                    sx += __shfl_xor_sync(0xffffffffu, sx, d, GZ);
-                    sy += __shfl_xor_sync(0xffffffffu, sy, d, GZ);
+#pragma unroll
+                    for (int n = 0; n < NQ; n++) {
+                        sx[n] += __shfl_xor_sync(0xffffffffu, sx[n], d, GZ);
+                        sy[n] += __shfl_xor_sync(0xffffffffu, sy[n], d, GZ);
+                    }
                 }
-                float2* out = q == 0 ? a.echo : q == 3 ? a.dT1 : a.dT2;
-                if (sub == 0 && vok) out[at] = make_float2(sx, sy);
+            } else {
+                // from part to part of a group: every lane adds, part i keeps it (straight-line code for the usual
+                // counts: a loop took 80 of 1850 ns per TR)
+                auto pass = [&](int i) __attribute__((always_inline)) {
+#pragma unroll
+                    for (int n = 0; n < NQ; n++) {
+                        float x = __shfl_up_sync(0xffffffffu, sx[n], 1, GZ), y = __shfl_up_sync(0xffffffffu, sy[n], 1, GZ);
+                        add_slots(n, x, y);
+                        if (part == i) sx[n] = x, sy[n] = y;
+                    }
+                };
+                pass(1);
+                if (parts > 2) {
+                    pass(2);
+                    for (int i = 3; i < parts; i++) pass(i);
+                }
+                auto merge = [&](int d) __attribute__((always_inline)) {  // the last parts of the groups
+                    const int from = (group ^ d) * parts + parts - 1;
+#pragma unroll
+                    for (int n = 0; n < NQ; n++) {
+                        sx[n] += __shfl_sync(0xffffffffu, sx[n], from, GZ);
+                        sy[n] += __shfl_sync(0xffffffffu, sy[n], from, GZ);
+                    }
+                };
+                if (split.lanes > 1) {
+                    if (split.lanes > 2) {
+                        for (int d = split.lanes / 2; d > 2; d /= 2) merge(d);
+                        merge(2);
+                    }
+                    merge(1);
+                }
+            }
+            if (sub == parts - 1 && vok) {
+#pragma unroll
+                for (int n = 0; n < NQ; n++) (n == 0 ? a.echo : n == 1 ? a.dT1 : a.dT2)[at] = make_float2(sx[n], sy[n]);
             }
             precess(E1_pr, E2_pr);
         }
@@ -395,18 +435,18 @@ __device__ __forceinline__ bool pssfp_real_rf(const PssfpArgs& a) {
 // One simulation (TAN: with its T1 and T2 tangents into a.dT1, a.dT2). Returns at once when the RF is not
 // real: the general kernel launched beside it runs then.
 template<int ZT, int GZ, bool TAN>
-__global__ void __launch_bounds__(128) pssfp_real_kernel(PssfpArgs a, HostAnswer ask) {
+__global__ void __launch_bounds__(128) pssfp_real_kernel(PssfpArgs a, PssfpSplit split, HostAnswer ask) {
     if (!TAN && a.skip != nullptr && *a.skip != 0) return;  // uniform over the grid
     answer_host(ask, pssfp_real_rf(a));
     if (!pssfp_real_rf(a)) return;
-    pssfp_real_tile<ZT, GZ, TAN>(a, blockIdx.x);
+    pssfp_real_tile<ZT, GZ, TAN>(a, split, blockIdx.x);
 }
 
 // Work-queue form for batches (see pssfp_queue_kernel): every job's RF is real.
 template<int ZT, int GZ, bool TAN>
 __global__ void __launch_bounds__(128) pssfp_real_queue_kernel(const PssfpArgs* __restrict__ jobs,
                                                                const int2* __restrict__ items, int nitems,
-                                                               int* __restrict__ head) {
+                                                               int* __restrict__ head, PssfpSplit split) {
     __shared__ PssfpArgs job;
     __shared__ int s_item;
     for (;;) {
@@ -417,7 +457,7 @@ __global__ void __launch_bounds__(128) pssfp_real_queue_kernel(const PssfpArgs* 
         const int2 w = items[it];
         if (threadIdx.x == 0) job = jobs[w.x];
         __syncthreads();
-        pssfp_real_tile<ZT, GZ, TAN>(job, w.y);
+        pssfp_real_tile<ZT, GZ, TAN>(job, split, w.y);
         __syncthreads();
     }
 }
@@ -426,8 +466,8 @@ __global__ void __launch_bounds__(128) pssfp_real_queue_kernel(const PssfpArgs* 
 
 struct PssfpRealKernels {
     int ZT, GZ;
-    void (*fn)(kernels::PssfpArgs, kernels::HostAnswer);
-    void (*queue)(const kernels::PssfpArgs*, const int2*, int, int*);
+    void (*fn)(kernels::PssfpArgs, kernels::PssfpSplit, kernels::HostAnswer);
+    void (*queue)(const kernels::PssfpArgs*, const int2*, int, int*, kernels::PssfpSplit);
 };
 // the real-RF value and tangent kernels of a layout (every layout of pssfp.cu has them)
 const PssfpRealKernels& pssfp_real_kernels(int ZT, int GZ);
