@@ -135,9 +135,12 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
     };
     std::vector<std::pair<Key, int>> keyed;
     std::map<Key, PssfpLaunch> pssfp_launch;
+    int64_t fisp_pairs = 0;  // (voxel, position) pairs of the FISP jobs with tangents
     std::map<std::pair<int, int>, int64_t> pssfp_voxels;  // of the real-RF jobs, by tangents and nz
     for (int j : members) {
         const auto& job = jobs[size_t(j)];
+        if (const auto* f = std::get_if<FISPSequence>(&job.sequence); f != nullptr && job.tangents)
+            fisp_pairs += int64_t(job.parameters.nvoxels) * f->sliceprofiles.size(0);
         const auto* seq = std::get_if<pSSFPSequence>(&job.sequence);
         if (seq != nullptr && job.parameters.nvoxels > 0 && pssfp_sequence_real_rf(ctx, *seq))
             pssfp_voxels[{job.tangents ? 1 : 0, int(seq->z.size())}] += job.parameters.nvoxels;
@@ -163,10 +166,12 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
             const bool states = fisp_real_covers(seq, tan != 0);
             const int real = (states || packed) && fisp_sequence_real_phases(ctx, seq) ? (states ? 2 : 1) : 0;
             if (real == 2) {
-                const int vb = tan ? fisp_real_tangent_tile_voxels(seq.max_state) : 32;
+                // (4 jobs of 100 to 1000 voxels, 8 states, with tangents: 70 us on one lane each, 31 us on 4)
+                const bool split = tan && fisp_real_tangent_split(fisp_pairs);
+                const int vb = tan ? fisp_real_tangent_tile_voxels(seq.max_state, split) : 32;
                 const int tiles = std::min(4, div_ceil(V, vb));
-                D = FispLaunch {0, tan ? fisp_real_tangent_queue_warps(seq.max_state, P, tiles)
-                                       : fisp_real_queue_warps(seq.max_state, P, tiles)};
+                D = FispLaunch {split ? 1 : 0, tan ? fisp_real_tangent_queue_warps(seq.max_state, split, P, tiles)
+                                                   : fisp_real_queue_warps(seq.max_state, P, tiles)};
             } else {
                 D.warps = std::max(1, std::min(D.warps, 8));
             }
@@ -213,7 +218,7 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
         if (fisp) {
             std::vector<kernels::FispArgs> args;
             const FispLaunch L {key.config, key.warps};
-            const int vb = g.states ? (g.tangent ? fisp_real_tangent_tile_voxels(g.cover) : 32)
+            const int vb = g.states ? (g.tangent ? fisp_real_tangent_tile_voxels(g.cover, g.config != 0) : 32)
                                     : (g.tangent ? fisp_tangent_tile_voxels(L) : fisp_tile_voxels(L));
             for (size_t q = 0; q < js.size(); q++) {
                 const auto& job = jobs[size_t(js[q])];
@@ -389,7 +394,7 @@ void SimulationBatch::Impl::enqueue(const Family& fam, cudaStream_t stream, int*
     const int dev = ctx.device();
     for (const auto& g : fam.sims) {
         if (g.states && g.tangent)
-            launch_fisp_real_tangent_queue(stream, dev, g.warps, g.cover, as<kernels::FispArgs>(g.args),
+            launch_fisp_real_tangent_queue(stream, dev, g.warps, g.cover, g.config != 0, as<kernels::FispArgs>(g.args),
                                            as<int2>(g.items), g.nitems, head_base + g.head);
         else if (g.fisp && g.tangent)
             launch_fisp_tangent_queue(stream, dev, FispLaunch {g.config, g.warps}, g.cover,

@@ -30,23 +30,26 @@ const RealLayout& covering(const RealLayout* layouts, int count, int N) {
         if (2 * layouts[i].KP * layouts[i].G + 1 >= N) return layouts[i];
     COMPAS_ERROR("no real-phase tangent layout holds the states");
 }
-const RealLayout& real_layout(int N) {
-    return covering(kLayouts, int(sizeof(kLayouts) / sizeof(kLayouts[0])), N);
+const RealLayout& real_layout(int N, bool split) {
+    return split ? covering(kSplitLayouts, 4, N) : covering(kLayouts, int(sizeof(kLayouts) / sizeof(kLayouts[0])), N);
 }
 
 }  // namespace
 
-int fisp_real_tangent_queue_warps(int N, int P, int64_t tiles) {
-    return fisp_real_warps(real_layout(N).warps, P, tiles);
+bool fisp_real_tangent_split(int64_t pairs) {
+    return pairs <= kRealSplitPairs;
 }
 
-int fisp_real_tangent_tile_voxels(int N) {
-    return 32 / real_layout(N).G;
+int fisp_real_tangent_queue_warps(int N, bool split, int P, int64_t tiles) {
+    return fisp_real_warps(real_layout(N, split).warps, P, tiles);
+}
+
+int fisp_real_tangent_tile_voxels(int N, bool split) {
+    return 32 / real_layout(N, split).G;
 }
 
 void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& a, const kernels::HostAnswer& ask) {
-    const RealLayout* layout = &real_layout(a.N);
-    if (int64_t(a.nvoxels) * a.P <= kRealSplitPairs) layout = &covering(kSplitLayouts, 4, a.N);
+    const RealLayout* layout = &real_layout(a.N, fisp_real_tangent_split(int64_t(a.nvoxels) * a.P));
     const int ntiles = div_ceil(a.nvoxels, 32 / layout->G);
     const int W = fisp_real_warps(layout->warps, a.P, div_ceil(ntiles, 148));
     const size_t smem = size_t(W) * layout->smem;
@@ -58,10 +61,10 @@ void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs&
     check_launch("fisp_real_kernel (tangents)");
 }
 
-void launch_fisp_real_tangent_queue(cudaStream_t stream, int device, int W, int max_state,
+void launch_fisp_real_tangent_queue(cudaStream_t stream, int device, int W, int max_state, bool split,
                                     const kernels::FispArgs* jobs, const int2* items, int nitems, int* head) {
     if (nitems <= 0) return;
-    const RealLayout& layout = real_layout(max_state);
+    const RealLayout& layout = real_layout(max_state, split);
     const void* fn = reinterpret_cast<const void*>(layout.queue);
     const size_t smem = size_t(W) * layout.smem;
     DeviceGuard guard(device);

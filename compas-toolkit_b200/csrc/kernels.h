@@ -67,11 +67,12 @@ void launch_fisp_real(const CompasContext& ctx, const kernels::FispArgs& args, c
 void launch_fisp_real_tangent(const CompasContext& ctx, const kernels::FispArgs& args, const kernels::HostAnswer& ask);
 // work queues: items of tiles of 32 voxels (tangents: fisp_real_tangent_tile_voxels), W warps per CTA
 int fisp_real_queue_warps(int N, int P, int64_t tiles);
-int fisp_real_tangent_queue_warps(int N, int P, int64_t tiles);
-int fisp_real_tangent_tile_voxels(int N);
+bool fisp_real_tangent_split(int64_t pairs);  // few (voxel, position) pairs in all: the states over 4 lanes
+int fisp_real_tangent_queue_warps(int N, bool split, int P, int64_t tiles);
+int fisp_real_tangent_tile_voxels(int N, bool split);
 void launch_fisp_real_queue(cudaStream_t stream, int device, int W, int max_state, const kernels::FispArgs* jobs,
                             const int2* items, int nitems, int* head);
-void launch_fisp_real_tangent_queue(cudaStream_t stream, int device, int W, int max_state,
+void launch_fisp_real_tangent_queue(cudaStream_t stream, int device, int W, int max_state, bool split,
                                     const kernels::FispArgs* jobs, const int2* items, int nitems, int* head);
 
 // value and T1/T2 tangents (forward mode) in one launch; L.config indexes the tangent layouts
