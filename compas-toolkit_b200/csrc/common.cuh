@@ -119,10 +119,6 @@ __device__ __forceinline__ void st_l2_hint(float2* ptr, float2 v, uint64_t polic
                  : "memory");
 }
 
-__device__ __forceinline__ void st_l2_hint(float* ptr, float v, uint64_t policy) {
-    asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(ptr), "f"(v), "l"(policy) : "memory");
-}
-
 // e^{i·2π·turns}: accurate for any magnitude of `turns` (sincospi reduces exactly)
 __device__ __forceinline__ float2 cis_turns(double turns) {
     double frac = turns - rint(turns);  // exact in FP64 for |turns| < 2^52

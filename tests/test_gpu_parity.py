@@ -232,11 +232,14 @@ def test_operators_match_reference_kernels(cb, ctx, ref_simulations, oracle):
 # pSSFP
 # ------------------------------------------------------------------------------------------------
 
+# phase 0: real RF, on the real-RF kernels (csrc/pssfp_real.cuh); else the general kernels
+@pytest.mark.parametrize("phase", [0.0, 0.4])
 @pytest.mark.parametrize("nz", [1, 5, 35])
-def test_pssfp_every_layout(cb, ctx, oracle, workloads, nz):
+def test_pssfp_every_layout(cb, ctx, oracle, workloads, nz, phase):
     rng = np.random.default_rng(nz)
     seq = workloads.pssfp_sequence(rng, 23, nrf=7, nz=nz)
     p = workloads.tissue(rng, 5, 20.0)
+    seq["rf"] = (seq["rf"] * np.exp(1j * phase * rng.uniform(-1, 1, len(seq["rf"])))).astype(np.complex64)
     params = cb.TissueParameters.from_soa(ctx, p)
     s = cb.pSSFPSequence.from_dict(ctx, seq)
     ref = oracle.pssfp(p, seq)
@@ -254,24 +257,26 @@ def test_pssfp_every_layout(cb, ctx, oracle, workloads, nz):
     assert tried > 0
 
 
-def test_pssfp_large_rotations(cb, ctx, oracle, workloads):
-    # flip angles of 120° per TR and strong off-resonance exercise the sincos branch
+@pytest.mark.parametrize("phase", [0.0, 0.4])
+def test_pssfp_large_rotations(cb, ctx, oracle, workloads, phase):
+    # flip angles of 120° per TR and strong off-resonance exercise the sincos branch (phase 0: the long series
+    # of the real-RF kernels)
     rng = np.random.default_rng(4)
     seq = workloads.pssfp_sequence(rng, 17, nrf=3, nz=9)
     seq["rf"] = (seq["rf"] * 3).astype(np.complex64)
     p = workloads.tissue(rng, 4, 20.0)
     p[3] *= 20
+    seq["rf"] = (seq["rf"] * np.exp(1j * phase * rng.uniform(-1, 1, 17))).astype(np.complex64)
     got = cb.simulate_magnetization(ctx, cb.TissueParameters.from_soa(ctx, p), cb.pSSFPSequence.from_dict(ctx, seq))
     assert oracle.rel_l2(got.to_numpy(), oracle.pssfp(p, seq)) < TOL_FP32
 
 
-@pytest.mark.parametrize("scale,phase", [(1, 0.0), (3, 0.0), (1, 0.4)])
+@pytest.mark.parametrize("scale,phase", [(1, 0.4), (3, 0.4), (1, 0.0)])
 def test_pssfp_packed_layouts_match_scalar_bits(cb, ctx, workloads, scale, phase):
     # a two-wide layout runs the scalar update's operations on pairs of isochromats and sums them in
     # the scalar order: the same bits as the scalar layout with as many isochromats per lane; at 3x
-    # the flip angles (and 20x the off-resonance) some pairs take the sincos branch. With a real RF
-    # train (phase 0) the packed layouts run their real-RF form, without the products of the zero
-    # axis component a_y: still the scalar bits (up to the sign of exact zeros)
+    # the flip angles (and 20x the off-resonance) some pairs take the sincos branch. (With a real RF train,
+    # phase 0, both run the real-RF kernel of that size.)
     rng = np.random.default_rng(12 + scale)
     seq = workloads.pssfp_sequence(rng, 19, nrf=5, nz=3)
     seq["rf"] = (seq["rf"] * scale * np.exp(1j * phase * rng.uniform(-1, 1, len(seq["rf"])))).astype(np.complex64)

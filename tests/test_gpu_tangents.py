@@ -148,11 +148,14 @@ def test_fisp_tangents_are_the_limit_of_the_reference_difference(cb, ctx, worklo
             assert err[1e-4] < err[1e-3] / 3, err
 
 
+# phase 0: real RF, on the real-RF kernels (csrc/pssfp_real.cuh); else the general kernels
+@pytest.mark.parametrize("phase", [0.0, 0.4])
 @pytest.mark.parametrize("nz", [1, 5, 35])
-def test_pssfp_tangents_every_layout(cb, ctx, oracle, workloads, nz):
+def test_pssfp_tangents_every_layout(cb, ctx, oracle, workloads, nz, phase):
     rng = np.random.default_rng(nz + 50)
     seqd = workloads.pssfp_sequence(rng, 21, nrf=7, nz=nz)
     p = workloads.tissue(rng, 5, 20.0)
+    seqd["rf"] = (seqd["rf"] * np.exp(1j * phase * rng.uniform(-1, 1, 21))).astype(np.complex64)
     params = cb.TissueParameters.from_soa(ctx, p)
     seq = cb.pSSFPSequence.from_dict(ctx, seqd)
     ref = {f: oracle.derivative_central(oracle.pssfp, p, seqd, i) for i, f in enumerate(("T1", "T2"))}
@@ -173,12 +176,12 @@ def test_pssfp_tangents_every_layout(cb, ctx, oracle, workloads, nz):
     assert tried > 0
 
 
-@pytest.mark.parametrize("scale,phase", [(1, 0.0), (3, 0.0), (1, 0.4)])
+@pytest.mark.parametrize("scale,phase", [(1, 0.4), (3, 0.4), (1, 0.0)])
 def test_pssfp_packed_tangents_match_scalar_bits(cb, ctx, workloads, scale, phase):
     # the two-wide tangent kernel runs the scalar tangent update's operations on pairs of isochromats:
     # m, ∂m/∂T1 and ∂m/∂T2 are the bits of the scalar layout with as many isochromats per lane (at 3x
-    # the flip angles and 20x the off-resonance, some pairs take the sincos branch; phase 0: the
-    # real-RF form)
+    # the flip angles and 20x the off-resonance, some pairs take the sincos branch; phase 0: both run the
+    # real-RF kernel of that size)
     rng = np.random.default_rng(30 + scale)
     seqd = workloads.pssfp_sequence(rng, 15, nrf=5, nz=3)
     seqd["rf"] = (seqd["rf"] * scale * np.exp(1j * phase * rng.uniform(-1, 1, len(seqd["rf"])))).astype(np.complex64)
@@ -203,13 +206,16 @@ def test_pssfp_packed_tangents_match_scalar_bits(cb, ctx, workloads, scale, phas
         cb.set_pssfp_launch(-1)
 
 
-def test_pssfp_tangents_large_rotations(cb, ctx, oracle, workloads):
-    # 3× the flip angles and 20× the off-resonance: the sincos branch of the rotation
+@pytest.mark.parametrize("phase", [0.0, 0.4])
+def test_pssfp_tangents_large_rotations(cb, ctx, oracle, workloads, phase):
+    # 3× the flip angles and 20× the off-resonance: the sincos branch of the rotation (phase 0: the long
+    # series of the real-RF kernels)
     rng = np.random.default_rng(4)
     seqd = workloads.pssfp_sequence(rng, 17, nrf=3, nz=9)
     seqd["rf"] = (seqd["rf"] * 3).astype(np.complex64)
     p = workloads.tissue(rng, 4, 20.0)
     p[3] *= 20
+    seqd["rf"] = (seqd["rf"] * np.exp(1j * phase * rng.uniform(-1, 1, 17))).astype(np.complex64)
     params = cb.TissueParameters.from_soa(ctx, p)
     got = cb.simulate_magnetization_tangents(ctx, params, cb.pSSFPSequence.from_dict(ctx, seqd))
     _check_tangents(cb, oracle, got, p, seqd, oracle.pssfp, oracle.pssfp(p, seqd))
