@@ -88,9 +88,9 @@ struct SimulationBatch::Impl {
         int config, warps, cover;  // layout, warps (FISP), max_state / nz
         bool real = false;         // every job's RF is real (FISP: RF and slice-profile phases)
         bool states = false;       // FISP: on the real-state kernels
-        PssfpLaunch pssfp {-1};
         Array<unsigned char> args;
         Array<unsigned char> items;
+        Array<unsigned char> orders;  // pSSFP with real RF: per job the order of its own layout's sum
         int nitems = 0;
         int head = 0;
     };
@@ -134,7 +134,6 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
         }
     };
     std::vector<std::pair<Key, int>> keyed;
-    std::map<Key, PssfpLaunch> pssfp_launch;
     int64_t fisp_pairs = 0;  // (voxel, position) pairs of the FISP jobs with tangents
     std::map<std::pair<int, int>, int64_t> pssfp_voxels;  // of the real-RF jobs, by tangents and nz
     for (int j : members) {
@@ -180,11 +179,10 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
             const auto& seq = std::get<pSSFPSequence>(job.sequence);
             const int nz = int(seq.z.size());
             // jobs with real RF form their own groups, on the real-RF kernels in the layout for all their
-            // voxels together (16 jobs of 100 to 4000 voxels and 9 z in each one's own: 678 us, in this 189 us)
+            // voxels together (16 jobs of 100 to 4000 voxels and 9 z in each one's own: 678 us, in this 279 us)
             const int real = pssfp_sequence_real_rf(ctx, seq) ? 1 : 0;
             const PssfpLaunch D = tuned_pssfp_launch(nz, real ? pssfp_voxels[{tan, nz}] : job.parameters.nvoxels, real != 0);
             keyed.push_back({Key {tan, D.config, 0, nz, real}, j});
-            pssfp_launch[keyed.back().first] = D;
         }
     }
     std::stable_sort(keyed.begin(), keyed.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
@@ -213,7 +211,6 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
         g.cover = key.cover;
         g.real = key.real != 0;
         g.states = fisp && key.real == 2;
-        if (!fisp) g.pssfp = pssfp_launch[key];
         std::vector<int> items;
         if (fisp) {
             std::vector<kernels::FispArgs> args;
@@ -240,6 +237,7 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
             g.args = upload_table(ctx, args);
         } else {
             std::vector<kernels::PssfpArgs> args;
+            std::vector<kernels::PssfpOrder> orders;
             const int vb = pssfp_tile_voxels(PssfpLaunch {key.config});
             for (size_t q = 0; q < js.size(); q++) {
                 const auto& job = jobs[size_t(js[q])];
@@ -250,12 +248,14 @@ void SimulationBatch::Impl::plan_simulation(Family& fam, bool fisp, const std::v
                     args.back().dT1 = reinterpret_cast<float2*>(dT1[size_t(js[q])].data());
                     args.back().dT2 = reinterpret_cast<float2*>(dT2[size_t(js[q])].data());
                 }
+                if (g.real) orders.push_back(pssfp_order(tuned_pssfp_launch(g.cover, V, true)));
                 for (int t = 0; t < div_ceil(V, vb); t++) {
                     items.push_back(int(q));
                     items.push_back(t);
                 }
             }
             g.args = upload_table(ctx, args);
+            if (g.real) g.orders = upload_table(ctx, orders);
         }
         g.nitems = int(items.size() / 2);
         g.items = upload_table(ctx, items);
@@ -407,11 +407,13 @@ void SimulationBatch::Impl::enqueue(const Family& fam, cudaStream_t stream, int*
             launch_fisp_queue(stream, dev, FispLaunch {g.config, g.warps}, g.cover, as<kernels::FispArgs>(g.args),
                               as<int2>(g.items), g.nitems, head_base + g.head, g.real);
         else if (g.tangent)
-            launch_pssfp_tangent_queue(stream, dev, g.pssfp, g.cover, as<kernels::PssfpArgs>(g.args),
-                                       as<int2>(g.items), g.nitems, head_base + g.head, g.real);
+            launch_pssfp_tangent_queue(stream, dev, PssfpLaunch {g.config}, g.cover, as<kernels::PssfpArgs>(g.args),
+                                       as<int2>(g.items), g.nitems, head_base + g.head,
+                                       g.real ? as<kernels::PssfpOrder>(g.orders) : nullptr);
         else
-            launch_pssfp_queue(stream, dev, g.pssfp, g.cover, as<kernels::PssfpArgs>(g.args),
-                               as<int2>(g.items), g.nitems, head_base + g.head, g.real);
+            launch_pssfp_queue(stream, dev, PssfpLaunch {g.config}, g.cover, as<kernels::PssfpArgs>(g.args),
+                               as<int2>(g.items), g.nitems, head_base + g.head,
+                               g.real ? as<kernels::PssfpOrder>(g.orders) : nullptr);
     }
     for (int j : fam.empty_signals)
         COMPAS_CUDA_CHECK(cudaMemsetAsync(signals[size_t(j)].data(), 0, signals[size_t(j)].nbytes(), stream));

@@ -62,10 +62,10 @@ struct PssfpArgs {
     const int* skip;  // one-simulation kernel: returns at once when *skip != 0 (null: never)
 };
 
-// The order in which the real-RF pSSFP kernels sum a voxel's isochromats: groups of `group`, `lanes` (a power of
-// two) of them (pssfp_real_tile)
-struct PssfpSplit {
-    int group, lanes;
+// The order in which a layout of the pSSFP kernels sums a voxel's isochromats: `zt` in order, `lanes` (a power of
+// two) of these as a tree
+struct PssfpOrder {
+    int zt = 0, lanes = 0;
 };
 
 // Where a one-simulation kernel of real phases or real RF tells the host whether the sequence is (a

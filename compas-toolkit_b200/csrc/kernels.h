@@ -94,8 +94,6 @@ void launch_fisp_tangent_queue(cudaStream_t stream, int device, FispLaunch L, in
 // ---- pSSFP ------------------------------------------------------------------------------
 struct PssfpLaunch {
     int config;  // index into the instantiated (ZT, GZ) layouts, -1 = default
-    // real-RF kernels: the order of the sum over the isochromats (kernels::PssfpSplit); 0: the layout's own
-    int group = 0, lanes = 0;
 };
 int pssfp_config_count();
 bool pssfp_config_info(int index, int* ZT, int* GZ);
@@ -103,8 +101,7 @@ bool pssfp_config_packed(int index);  // two-wide layout: ZT/2 pairs of isochrom
 PssfpLaunch pssfp_default_launch(int nz, int64_t nvoxels);
 PssfpLaunch pssfp_real_default_launch(int nz, int64_t nvoxels);
 // real: the layout of the real-RF kernels (pssfp_real.cuh), which differ from the general ones' only in
-// the default. All defaults for one nz sum the isochromats in one order, so the echoes do not depend on nvoxels;
-// an explicit override sums in its own.
+// the default
 PssfpLaunch tuned_pssfp_launch(int nz, int64_t nvoxels, bool real = false);
 void launch_pssfp(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
                   const pSSFPSequence& seq, cfloat* echo, int64_t echo_stride, PssfpLaunch L,
@@ -117,13 +114,15 @@ int pssfp_tile_voxels(PssfpLaunch L);
 void launch_pssfp_tangent(const CompasContext& ctx, const TissueParameters& params, int voxel_begin, int nvoxels,
                           const pSSFPSequence& seq, cfloat* echo, cfloat* dT1, cfloat* dT2, int64_t echo_stride,
                           PssfpLaunch L);
-// work-queue launches over (job, tile) items of pSSFP jobs that all use layout L; `real`: every job's
-// RF is real (pssfp_sequence_real_rf), which the kernels of pssfp_real.cuh run
+// work-queue launches over (job, tile) items of pSSFP jobs that all use layout L; `real`: not null when every job's
+// RF is real (pssfp_sequence_real_rf), which the kernels of pssfp_real.cuh run: per job the order of the sum of
+// its own layout (pssfp_order), so that its echoes are those of a call of its own
+kernels::PssfpOrder pssfp_order(PssfpLaunch L);
 void launch_pssfp_tangent_queue(cudaStream_t stream, int device, PssfpLaunch L, int nz,
                                 const kernels::PssfpArgs* jobs, const int2* items, int nitems, int* head,
-                                bool real = false);
+                                const kernels::PssfpOrder* real);
 void launch_pssfp_queue(cudaStream_t stream, int device, PssfpLaunch L, int nz, const kernels::PssfpArgs* jobs,
-                        const int2* items, int nitems, int* head, bool real = false);
+                        const int2* items, int nitems, int* head, const kernels::PssfpOrder* real);
 // whether every RF sample of the sequence (RF train × waveform) is real, read back from its rotation
 // table: synchronises the context's stream the first time (not while it is captured)
 bool pssfp_sequence_real_rf(const CompasContext& ctx, const pSSFPSequence& seq);

@@ -660,40 +660,24 @@ PssfpLaunch pssfp_default_launch(int nz, int64_t nvoxels) {
 // fall to it. So many voxels take the fewest slots and few voxels more lanes: 35 z of 15 RF samples and 100
 // TRs, 9 isochromats on 4 lanes / 5 on 8 / 3 on 16, in us: 279 / 229 / 212 at 2500 voxels, 279 / 234 / 272
 // at 4096, 362 / 413 / 446 at 8000. On a tie the fewer slots, then the fewer lanes. At most 10
-// isochromats per lane: the tangents of more do not fit the registers. The layout of many voxels sets the order of
-// the sum over the isochromats, and the others are those that can keep it (pssfp_real_tile): its lanes'
-// isochromats dealt out to several lanes each.
+// isochromats per lane: the tangents of more do not fit the registers.
 PssfpLaunch pssfp_real_default_launch(int nz, int64_t nvoxels) {
+    int best = -1;
+    double best_time = 0.0;
     auto slots = [](int i) { return kPssfpConfigs[i].ZT * kPssfpConfigs[i].GZ; };
-    auto least = [&](auto eligible, auto estimate) {
-        int best = -1;
-        double best_time = 0.0;
-        for (int i = 0; i < pssfp_config_count(); i++) {
-            const auto& c = kPssfpConfigs[i];
-            if (c.ZT > 10 || slots(i) < nz || !eligible(c)) continue;
-            const double time = estimate(c);
-            const bool tie = best >= 0 && std::abs(time - best_time) < 1e-9 * time;
-            if (best < 0 || (!tie && time < best_time) ||
-                (tie && (slots(i) < slots(best) || (slots(i) == slots(best) && c.GZ < kPssfpConfigs[best].GZ)))) {
-                best = i;
-                best_time = time;
-            }
+    for (int i = 0; i < pssfp_config_count(); i++) {
+        const auto& c = kPssfpConfigs[i];
+        if (slots(i) < nz || c.ZT > 10) continue;
+        const double warps = double(nvoxels) * c.GZ / (32.0 * 4 * 148);
+        const double time = std::max(155.0 + 21.0 * c.ZT, (25.0 + 17.0 * c.ZT) * (warps < 8.0 ? std::ceil(warps) : warps));
+        const bool tie = best >= 0 && std::abs(time - best_time) < 1e-9 * time;
+        if (best < 0 || (!tie && time < best_time) ||
+            (tie && (slots(i) < slots(best) || (slots(i) == slots(best) && c.GZ < kPssfpConfigs[best].GZ)))) {
+            best = i;
+            best_time = time;
         }
-        return best;
-    };
-    const int many = least([](const PssfpConfig&) { return true; }, [](const PssfpConfig& c) { return c.GZ * (25.0 + 17.0 * c.ZT); });
-    if (many < 0) return pssfp_default_launch(nz, nvoxels);
-    const int group = kPssfpConfigs[many].ZT, lanes = kPssfpConfigs[many].GZ;
-    const int best = least(
-        [&](const PssfpConfig& c) {
-            const int parts = div_ceil(group, c.ZT);
-            return parts == 1 ? c.ZT == group && c.GZ == lanes : lanes * parts <= c.GZ;
-        },
-        [&](const PssfpConfig& c) {
-            const double warps = double(nvoxels) * c.GZ / (32.0 * 4 * 148);
-            return std::max(155.0 + 21.0 * c.ZT, (25.0 + 17.0 * c.ZT) * (warps < 8.0 ? std::ceil(warps) : warps));
-        });
-    return PssfpLaunch {best, group, lanes};
+    }
+    return best < 0 ? pssfp_default_launch(nz, nvoxels) : PssfpLaunch {best};
 }
 
 kernels::PssfpArgs pssfp_args(const CompasContext& ctx, const TissueParameters& params, int voxel_begin,
@@ -770,10 +754,6 @@ const PssfpConfig& checked_config(PssfpLaunch L, int nz) {
     return cfg;
 }
 constexpr int kPssfpThreads = 128;
-kernels::PssfpSplit pssfp_split(PssfpLaunch L) {
-    if (L.group > 0) return {L.group, L.lanes};
-    return {kPssfpConfigs[L.config].ZT, kPssfpConfigs[L.config].GZ};
-}
 unsigned pssfp_grid(int nvoxels, int GZ) {
     return unsigned((int64_t(nvoxels) * GZ + kPssfpThreads - 1) / kPssfpThreads);
 }
@@ -801,41 +781,46 @@ void launch_pssfp(const CompasContext& ctx, const TissueParameters& params, int 
         check_launch("pssfp_kernel");
     }
     if (form.real == 0) return;
-    const PssfpLaunch R = tuned_pssfp_launch(nz, nvoxels, true);
-    const auto& real = checked_config(R, nz);
-    pssfp_real_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a, pssfp_split(R),
-                                                                                                       form.ask);
+    const auto& real = checked_config(tuned_pssfp_launch(nz, nvoxels, true), nz);
+    pssfp_real_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a, form.ask);
     check_launch("pssfp_real_kernel");
 }
 
 namespace {
-void launch_queue(cudaStream_t stream, int device, PssfpLaunch L, PssfpQueueKernel general, const PssfpRealKernels* real,
-                  const kernels::PssfpArgs* jobs, const int2* items, int nitems, int* head) {
+void launch_queue(cudaStream_t stream, int device, PssfpQueueKernel general, const PssfpRealKernels* real,
+                  const kernels::PssfpArgs* jobs, const int2* items, int nitems, int* head, const kernels::PssfpOrder* own) {
     DeviceGuard guard(device);
     const void* fn = real != nullptr ? reinterpret_cast<const void*>(real->queue) : reinterpret_cast<const void*>(general);
     int per_sm = 1, sms = 148;
     COMPAS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPssfpThreads, 0));
     COMPAS_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int grid = std::max(1, std::min(nitems, std::max(1, per_sm) * sms));
-    if (real != nullptr) real->queue<<<grid, kPssfpThreads, 0, stream>>>(jobs, items, nitems, head, pssfp_split(L));
+    if (real != nullptr) real->queue<<<grid, kPssfpThreads, 0, stream>>>(jobs, items, nitems, head, own);
     else general<<<grid, kPssfpThreads, 0, stream>>>(jobs, items, nitems, head);
     check_launch("pssfp_queue_kernel");
 }
 }  // namespace
 
+kernels::PssfpOrder pssfp_order(PssfpLaunch L) {
+    COMPAS_CHECK(L.config >= 0 && L.config < pssfp_config_count());
+    return {kPssfpConfigs[L.config].ZT, kPssfpConfigs[L.config].GZ};
+}
+
 void launch_pssfp_queue(cudaStream_t stream, int device, PssfpLaunch L, int nz, const kernels::PssfpArgs* jobs,
-                        const int2* items, int nitems, int* head, bool real) {
+                        const int2* items, int nitems, int* head, const kernels::PssfpOrder* real) {
     if (nitems <= 0) return;
     const auto& cfg = checked_config(L, nz);
-    launch_queue(stream, device, L, cfg.queue, real ? &pssfp_real_kernels(cfg.ZT, cfg.GZ) : nullptr, jobs, items, nitems, head);
+    launch_queue(stream, device, cfg.queue, real != nullptr ? &pssfp_real_kernels(cfg.ZT, cfg.GZ) : nullptr, jobs, items, nitems,
+                 head, real);
 }
 
 void launch_pssfp_tangent_queue(cudaStream_t stream, int device, PssfpLaunch L, int nz,
-                                const kernels::PssfpArgs* jobs, const int2* items, int nitems, int* head, bool real) {
+                                const kernels::PssfpArgs* jobs, const int2* items, int nitems, int* head,
+                                const kernels::PssfpOrder* real) {
     if (nitems <= 0) return;
     const auto& cfg = checked_config(L, nz);
-    launch_queue(stream, device, L, cfg.tangent_queue, real ? &pssfp_real_tangent_kernels(cfg.ZT, cfg.GZ) : nullptr, jobs, items,
-                 nitems, head);
+    launch_queue(stream, device, cfg.tangent_queue, real != nullptr ? &pssfp_real_tangent_kernels(cfg.ZT, cfg.GZ) : nullptr, jobs,
+                 items, nitems, head, real);
 }
 
 bool pssfp_sequence_real_rf(const CompasContext& ctx, const pSSFPSequence& seq) {
@@ -875,10 +860,8 @@ void launch_pssfp_tangent(const CompasContext& ctx, const TissueParameters& para
         check_launch("pssfp_tangent_kernel");
     }
     if (form.real == 0) return;
-    const PssfpLaunch R = tuned_pssfp_launch(nz, nvoxels, true);
-    const auto& real = checked_config(R, nz);
-    pssfp_real_tangent_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(
-        a, pssfp_split(R), form.ask);
+    const auto& real = checked_config(tuned_pssfp_launch(nz, nvoxels, true), nz);
+    pssfp_real_tangent_kernels(real.ZT, real.GZ).fn<<<pssfp_grid(nvoxels, real.GZ), kPssfpThreads, 0, ctx.stream()>>>(a, form.ask);
     check_launch("pssfp_real_kernel (tangents)");
 }
 

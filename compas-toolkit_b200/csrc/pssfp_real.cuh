@@ -190,24 +190,19 @@ __device__ __forceinline__ void real_precess(T (&v)[TAN ? 9 : 3], T c, T sn, T n
     }
 }
 
-// One tile (128/GZ voxels) of a simulation: GZ lanes per voxel, up to ZT isochromats per lane, slots p and
-// p + ZT/2 in a pair, an odd last slot by itself.
-//
-// The echo is the sum over the isochromats in an order that belongs to their number alone: one after the
-// other within the groups of split.group, and those as a tree over the split.lanes groups. That is the
-// order of the layout of many voxels, a group to a lane. A layout of more lanes deals a group out to `parts`
-// neighbouring lanes in chunks of ZT and passes the running sum along them. What a lane needs follows from all the
-// isochromats of its voxel, so the echoes are the same bits in every layout: one simulation takes the
-// layout for its voxels, a batch the one for all its voxels.
-template<int ZT, int GZ, bool TAN>
-__device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const PssfpSplit split, const int tile) {
+// One tile (128/GZ voxels) of a simulation: GZ lanes per voxel, ZT isochromats per lane, slots p and
+// p + ZT/2 in a pair, an odd last slot by itself. The isochromats evolve in the same bits in every layout (what a
+// voxel needs follows from all of them); the echo sums a lane's slots in order and the lanes as a tree.
+// QUEUE: the layout is the batch's, the sum that of `own`, the job's layout in a call of its own, where the two differ:
+// through shared memory (`sums`, ZT entries per thread), own.zt isochromats in order and own.lanes of these as the
+// same tree.
+template<int ZT, int GZ, bool TAN, bool QUEUE = false>
+__device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const int tile, const PssfpOrder own = {},
+                                                float2* sums = nullptr) {
     constexpr int ZP = ZT / 2, ODD = ZT % 2, ZA = ZP > 0 ? ZP : 1, NV = TAN ? 9 : 3;
     const int lane = threadIdx.x & 31;
     const int sub = lane % GZ;
-    const int parts = GZ == 1 ? 1 : (split.group + ZT - 1) / ZT;
-    const int group = GZ == 1 ? 0 : sub / parts, part = GZ == 1 ? 0 : sub % parts;
-    const int first = group * split.group + part * ZT;  // the lane's first isochromat
-    const int count = min(min(ZT, split.group - part * ZT), a.nz - first);  // and their number (or none, ≤ 0)
+    const int first = sub * ZT, count = a.nz - first;  // the lane's first isochromat; its slots below count hold one
     const int vloc = (tile * blockDim.x + threadIdx.x) / GZ;
     const bool vok = vloc < a.nvoxels;
     const int64_t vcol = a.voxel_begin + (vok ? vloc : a.nvoxels - 1);
@@ -347,76 +342,58 @@ __device__ __forceinline__ void pssfp_real_tile(const PssfpArgs& a, const PssfpS
             pulse_of(t + 1);
             precess(E1_first, E2_first);
             const int64_t at = int64_t(t) * a.echo_stride + a.voxel_begin + vloc;
-            constexpr int NQ = NV / 3;
-            float sx[NQ], sy[NQ];
-            auto add_slots = [&](int n, float& x, float& y) __attribute__((always_inline)) {  // in order
-                const int q = 3 * n;
+#pragma unroll
+            for (int q = 0; q < NV; q += 3) {
+                float2* out = q == 0 ? a.echo : q == 3 ? a.dT1 : a.dT2;
+                if (QUEUE && (own.zt != ZT || own.lanes != GZ)) {
+                    float2* m = sums + (threadIdx.x / GZ) * (ZT * GZ);  // the voxel's isochromats
+#pragma unroll
+                    for (int p = 0; p < ZP; p++) {
+                        if (p < count) m[first + p] = make_float2(P[p][q].x, P[p][q + 1].x);
+                        if (p + ZP < count) m[first + p + ZP] = make_float2(P[p][q].y, P[p][q + 1].y);
+                    }
+                    if (ODD && 2 * ZP < count) m[first + 2 * ZP] = make_float2(O[q], O[q + 1]);
+                    __syncwarp();
+                    const int used = (a.nz + own.zt - 1) / own.zt;  // the other lanes' sums are zero
+                    for (int v = sub; v < used; v += GZ) {
+                        float2 s = make_float2(0.f, 0.f);
+                        for (int z = v * own.zt; z < min((v + 1) * own.zt, a.nz); z++) s.x += m[z].x, s.y += m[z].y;
+                        m[v * own.zt] = s;
+                    }
+                    for (int d = own.lanes / 2; d > 0; d /= 2) {
+                        __syncwarp();
+                        for (int v = sub; v < d && v + d < used; v += GZ) {
+                            float2 &s = m[v * own.zt], t = m[(v + d) * own.zt];
+                            s.x += t.x, s.y += t.y;
+                        }
+                    }
+                    if (sub == 0 && vok) out[at] = m[0];
+                    __syncwarp();
+                    continue;
+                }
+                float sx = 0.0f, sy = 0.0f;  // over the slots in order
 #pragma unroll
                 for (int p = 0; p < ZP; p++)
                     if (p < count) {
-                        x += P[p][q].x;
-                        y += P[p][q + 1].x;
+                        sx += P[p][q].x;
+                        sy += P[p][q + 1].x;
                     }
 #pragma unroll
                 for (int p = 0; p < ZP; p++)
                     if (p + ZP < count) {
-                        x += P[p][q].y;
-                        y += P[p][q + 1].y;
+                        sx += P[p][q].y;
+                        sy += P[p][q + 1].y;
                     }
                 if (ODD && 2 * ZP < count) {
-                    x += O[q];
-                    y += O[q + 1];
+                    sx += O[q];
+                    sy += O[q + 1];
                 }
-            };
-#pragma unroll
-            for (int n = 0; n < NQ; n++) {
-                sx[n] = sy[n] = 0.0f;
-                add_slots(n, sx[n], sy[n]);
-            }
-            if (GZ == 1 || parts == 1) {
 #pragma unroll
                 for (int d = GZ / 2; d > 0; d /= 2) {
-#pragma unroll
-                    for (int n = 0; n < NQ; n++) {
-                        sx[n] += __shfl_xor_sync(0xffffffffu, sx[n], d, GZ);
-                        sy[n] += __shfl_xor_sync(0xffffffffu, sy[n], d, GZ);
-                    }
+                    sx += __shfl_xor_sync(0xffffffffu, sx, d, GZ);
+                    sy += __shfl_xor_sync(0xffffffffu, sy, d, GZ);
                 }
-            } else {
-                // from part to part of a group: every lane adds, part i keeps it (straight-line code for the usual
-                // counts: a loop took 80 of 1850 ns per TR)
-                auto pass = [&](int i) __attribute__((always_inline)) {
-#pragma unroll
-                    for (int n = 0; n < NQ; n++) {
-                        float x = __shfl_up_sync(0xffffffffu, sx[n], 1, GZ), y = __shfl_up_sync(0xffffffffu, sy[n], 1, GZ);
-                        add_slots(n, x, y);
-                        if (part == i) sx[n] = x, sy[n] = y;
-                    }
-                };
-                pass(1);
-                if (parts > 2) {
-                    pass(2);
-                    for (int i = 3; i < parts; i++) pass(i);
-                }
-                auto merge = [&](int d) __attribute__((always_inline)) {  // the last parts of the groups
-                    const int from = (group ^ d) * parts + parts - 1;
-#pragma unroll
-                    for (int n = 0; n < NQ; n++) {
-                        sx[n] += __shfl_sync(0xffffffffu, sx[n], from, GZ);
-                        sy[n] += __shfl_sync(0xffffffffu, sy[n], from, GZ);
-                    }
-                };
-                if (split.lanes > 1) {
-                    if (split.lanes > 2) {
-                        for (int d = split.lanes / 2; d > 2; d /= 2) merge(d);
-                        merge(2);
-                    }
-                    merge(1);
-                }
-            }
-            if (sub == parts - 1 && vok) {
-#pragma unroll
-                for (int n = 0; n < NQ; n++) (n == 0 ? a.echo : n == 1 ? a.dT1 : a.dT2)[at] = make_float2(sx[n], sy[n]);
+                if (sub == 0 && vok) out[at] = make_float2(sx, sy);
             }
             precess(E1_pr, E2_pr);
         }
@@ -435,18 +412,19 @@ __device__ __forceinline__ bool pssfp_real_rf(const PssfpArgs& a) {
 // One simulation (TAN: with its T1 and T2 tangents into a.dT1, a.dT2). Returns at once when the RF is not
 // real: the general kernel launched beside it runs then.
 template<int ZT, int GZ, bool TAN>
-__global__ void __launch_bounds__(128) pssfp_real_kernel(PssfpArgs a, PssfpSplit split, HostAnswer ask) {
+__global__ void __launch_bounds__(128) pssfp_real_kernel(PssfpArgs a, HostAnswer ask) {
     if (!TAN && a.skip != nullptr && *a.skip != 0) return;  // uniform over the grid
     answer_host(ask, pssfp_real_rf(a));
     if (!pssfp_real_rf(a)) return;
-    pssfp_real_tile<ZT, GZ, TAN>(a, split, blockIdx.x);
+    pssfp_real_tile<ZT, GZ, TAN>(a, blockIdx.x);
 }
 
-// Work-queue form for batches (see pssfp_queue_kernel): every job's RF is real.
+// Work-queue form for batches (see pssfp_queue_kernel): every job's RF is real; own: each job's own order of the sum.
 template<int ZT, int GZ, bool TAN>
 __global__ void __launch_bounds__(128) pssfp_real_queue_kernel(const PssfpArgs* __restrict__ jobs,
                                                                const int2* __restrict__ items, int nitems,
-                                                               int* __restrict__ head, PssfpSplit split) {
+                                                               int* __restrict__ head, const PssfpOrder* __restrict__ own) {
+    __shared__ float2 sums[128 * ZT];
     __shared__ PssfpArgs job;
     __shared__ int s_item;
     for (;;) {
@@ -457,7 +435,7 @@ __global__ void __launch_bounds__(128) pssfp_real_queue_kernel(const PssfpArgs* 
         const int2 w = items[it];
         if (threadIdx.x == 0) job = jobs[w.x];
         __syncthreads();
-        pssfp_real_tile<ZT, GZ, TAN>(job, split, w.y);
+        pssfp_real_tile<ZT, GZ, TAN, true>(job, w.y, own[w.x], sums);
         __syncthreads();
     }
 }
@@ -466,8 +444,8 @@ __global__ void __launch_bounds__(128) pssfp_real_queue_kernel(const PssfpArgs* 
 
 struct PssfpRealKernels {
     int ZT, GZ;
-    void (*fn)(kernels::PssfpArgs, kernels::PssfpSplit, kernels::HostAnswer);
-    void (*queue)(const kernels::PssfpArgs*, const int2*, int, int*, kernels::PssfpSplit);
+    void (*fn)(kernels::PssfpArgs, kernels::HostAnswer);
+    void (*queue)(const kernels::PssfpArgs*, const int2*, int, int*, const kernels::PssfpOrder*);
 };
 // the real-RF value and tangent kernels of a layout (every layout of pssfp.cu has them)
 const PssfpRealKernels& pssfp_real_kernels(int ZT, int GZ);

@@ -119,33 +119,29 @@ def test_large_angles_and_masked_voxels_against_oracle(cb, ctx, oracle):
 
 
 @pytest.mark.parametrize("nz", [1, 3, 5, 9, 12, 20, 35, 48, 64])
-def test_bits_do_not_depend_on_the_layout(cb, ctx, nz):
-    # the layouts for many and for few voxels and the one that a batch takes for all its jobs: the same bits, with
-    # voxels of every loop among them
+def test_batch_bits_are_those_of_each_job_alone(cb, ctx, oracle, nz):
+    # a batch takes one layout for all its voxels and sums each job's isochromats in the order of the job's own
+    # layout, for many or few voxels; jobs with voxels of every loop. Between the layouts only that order differs.
     rng = np.random.default_rng([8, nz])
     seq = W.pssfp_sequence(rng, 9, nrf=4, nz=nz)
     seq["gz"] = (0.09, seq["gz"][1], seq["gz"][2])
     p = W.tissue_voxels(rng, 40001, 22.4)
     p[3, ::11] = rng.uniform(-3000.0, 3000.0, p[3, ::11].size)
     p[3, 5::301] = 5000.0
-    p[1, 3::17] = 1e-5
     s = cb.pSSFPSequence.from_dict(ctx, seq)
-
-    def run(params):
-        t = cb.simulate_magnetization_tangents(ctx, params, s)
-        return [cb.simulate_magnetization(ctx, params, s).to_numpy()] + [t[k].to_numpy() for k in ("echos", "T1", "T2")]
-
-    cuts = [(0, 40001), (100, 9100), (5000, 8000), (300, 1500), (200, 260)]
+    cuts = [(0, 40001), (100, 9100), (5000, 8000), (300, 1500), (200, 260), (7, 8)]
     params = [cb.TissueParameters.from_soa(ctx, np.ascontiguousarray(p[:, a:b])) for a, b in cuts]
-    many = run(params[0])
-    assert np.array_equal(many[0], many[1], equal_nan=True)
-    for (a, b), q in zip(cuts[1:], params[1:]):
-        for x, y in zip(run(q), many):
-            assert np.array_equal(x, y[:, a:b], equal_nan=True), (a, b)
-    batch = cb.SimulationBatch(ctx, [(q, s, None, None) for q in params[1:]], tangents=[False, True, True, False])
-    batch.run()
-    ctx.synchronize()
-    for i, (a, b) in enumerate(cuts[1:]):
-        assert np.array_equal(batch.echos(i).to_numpy(), many[0][:, a:b], equal_nan=True)
-        if i in (1, 2):
-            assert np.array_equal(batch.derivative(i, "T2").to_numpy(), many[3][:, a:b], equal_nan=True)
+    many = cb.simulate_magnetization(ctx, params[0], s).to_numpy()
+    for jobs in (range(6), range(1, 6), (3, 5), (4, 5)):
+        tangents = [i % 2 == 1 for i in jobs]
+        batch = cb.SimulationBatch(ctx, [(params[i], s, None, None) for i in jobs], tangents=tangents)
+        batch.run()
+        ctx.synchronize()
+        for n, (i, tan) in enumerate(zip(jobs, tangents)):
+            alone = cb.simulate_magnetization_tangents(ctx, params[i], s) if tan else None
+            echos = (alone["echos"] if tan else cb.simulate_magnetization(ctx, params[i], s)).to_numpy()
+            assert np.array_equal(batch.echos(n).to_numpy(), echos), (nz, i)
+            assert oracle.rel_l2(echos, many[:, cuts[i][0]:cuts[i][1]]) < 1e-6
+            if tan:
+                for f in ("T1", "T2"):
+                    assert np.array_equal(batch.derivative(n, f).to_numpy(), alone[f].to_numpy()), (nz, i, f)
