@@ -315,6 +315,7 @@ void SimulationBatch::Impl::plan_signal(Family& fam, const std::vector<int>& mem
                                                echos[size_t(e.job)].data(), job.coil_sensitivities.data(), C,
                                                cartesian_geom(t));
             a.vchunk = e.plan.vchunk;
+            a.chunk_log2 = e.plan.chunk_log2;
             a.status = ctx.status_word();
             const TcTables tables = tc_tables(V, t.nreadouts, t.samples_per_readout, C, false);
             Array<unsigned char> scratch({tables.bytes}, dev, ctx.stream());

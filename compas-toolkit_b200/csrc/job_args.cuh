@@ -111,6 +111,7 @@ struct TcArgs {
     int R, S, C;
     float dt, dk_re, dk_im;
     int vchunk;           // voxels per split
+    int chunk_log2;       // stages per accumulation chunk, 2^chunk_log2
     float2* out;          // [splits][C][R][S]
     unsigned int* status;
     // tables written by the prep kernel:

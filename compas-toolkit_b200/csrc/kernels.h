@@ -181,6 +181,7 @@ bool tensor_cores_available(int device);
 struct TcPlan {
     int ntiles, mtiles, splits, vchunk;  // pair tiles, readout tiles, voxel splits, voxels per split
     int nr;                              // readouts per tile
+    int chunk_log2;                      // stages per accumulation chunk, 2^chunk_log2
     int64_t ctas;                        // CTAs of the contraction (CTA pairs × 2)
 };
 // readouts per tile of the Cartesian contraction: a multiple of 16 up to 256, the fewest tiles,

@@ -63,9 +63,10 @@ constexpr int TC_BH_BYTES = (TC_N / 2) * TC_K * 2;  // 16 KB per hi/lo plane: th
 constexpr int TC_STAGE_BYTES = 2 * TC_A_BYTES + 2 * TC_BH_BYTES;
 constexpr int TC_SMEM = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
 // TMEM of a CTA: the MMA accumulator (columns 0 .. nr-1) and the running FP32 sum of the finished
-// accumulation chunks (columns TC_SUM_COL ..); a chunk is TC_CHUNK_STAGES stages = 512 K16 steps
+// accumulation chunks (columns TC_SUM_COL ..); a chunk is 2^chunk_log2 stages (tc_plan), at most
+// 2^TC_CHUNK_LOG2 = 512 K16 steps
 constexpr int TC_TMEM_COLS = 512, TC_SUM_COL = 256;
-constexpr int TC_CHUNK_STAGES = 128;
+constexpr int TC_CHUNK_LOG2 = 7;
 static_assert(TC_PAIRS / 2 == (TC_B_THREADS / 16) * TC_PPG, "a CTA's producer groups cover half the pair tile");
 static_assert((TC_PAIRS / 2) * (2 * 256 + 2) * 4 <= TC_STAGES * TC_STAGE_BYTES, "output tile fits the stage buffers");
 
@@ -185,7 +186,9 @@ __global__ void __launch_bounds__(256) tc_pack_a_kernel(TcArgs a) {
 // barriers and the leader's commits arrive on both. D per CTA: 128 rows (64 pairs × re/im) × nr
 // readout columns. Shared by the one-operation kernel and the batched kernel, so both give
 // bit-identical results.
-template<bool JAC>
+// SHORT: accumulation chunks of a.chunk_log2, else all of 2^TC_CHUNK_LOG2 stages (known to the compiler: the signal of
+// the MR-STAT slice took 0.8 % longer with the argument)
+template<bool JAC, bool SHORT>
 __device__ __forceinline__ void tc_tile(const TcArgs& a, const int bx, const int by, const int bz,
                                         unsigned char* smem_raw) {
     constexpr int TERMS = JAC ? 2 : 1;            // complex terms per voxel along K
@@ -207,6 +210,7 @@ __device__ __forceinline__ void tc_tile(const TcArgs& a, const int bx, const int
     const int r0 = by * a.nr;
     const int v_begin = bz * a.vchunk;
     const int v_end = min(a.nvoxels, v_begin + a.vchunk);
+    const int chunk_log2 = SHORT ? a.chunk_log2 : TC_CHUNK_LOG2, chunk_mask = (1 << chunk_log2) - 1;
     const int nstages = max(1, (v_end - v_begin + VPS - 1) / VPS);
     const int npairs = a.C * a.S;
 
@@ -258,11 +262,11 @@ __device__ __forceinline__ void tc_tile(const TcArgs& a, const int bx, const int
             const uint32_t idesc = tc::idesc_bf16_f32(2 * TC_M, a.nr);
             for (int it = 0; it < nstages; it++) {
                 const int buf = it % TC_STAGES;
-                if (it > 0 && it % TC_CHUNK_STAGES == 0) {
+                if (it > 0 && (it & chunk_mask) == 0) {
                     // end of an accumulation chunk: once its MMAs complete, the producers of both
                     // CTAs add the accumulator into the running sum; the next chunk starts from 0
                     tc::mma_commit_pair(cdone);
-                    if (!tc::mbar_wait(drained, ((it / TC_CHUNK_STAGES) - 1) & 1, a.status)) *abort_flag = 1;
+                    if (!tc::mbar_wait(drained, ((it >> chunk_log2) - 1) & 1, a.status)) *abort_flag = 1;
                     if (*(volatile int*)abort_flag) break;
                     tc::tc_fence_after();
                 }
@@ -279,7 +283,7 @@ __device__ __forceinline__ void tc_tile(const TcArgs& a, const int bx, const int
                     const uint32_t koff = ks * 32;  // 16 bf16 = 32 bytes along K inside the swizzle atom
                     const uint64_t dah = tc::sw128_kmajor_desc(ah + koff), dal = tc::sw128_kmajor_desc(al + koff);
                     const uint64_t dbh = tc::sw128_kmajor_desc(bh + koff), dbl = tc::sw128_kmajor_desc(bl + koff);
-                    tc::mma_bf16_pair(tmem, dah, dbh, idesc, (it % TC_CHUNK_STAGES > 0 || ks > 0) ? 1u : 0u);
+                    tc::mma_bf16_pair(tmem, dah, dbh, idesc, ((it & chunk_mask) > 0 || ks > 0) ? 1u : 0u);
                     tc::mma_bf16_pair(tmem, dah, dbl, idesc, 1u);
                     tc::mma_bf16_pair(tmem, dal, dbh, idesc, 1u);
                 }
@@ -333,11 +337,11 @@ __device__ __forceinline__ void tc_tile(const TcArgs& a, const int bx, const int
         for (int it = 0; it < nstages; it++) {
             const int buf = it % TC_STAGES;
             const int vbase = v_begin + it * VPS + VPH * hq;
-            if (it > 0 && it % TC_CHUNK_STAGES == 0) {
+            if (it > 0 && (it & chunk_mask) == 0) {
                 // fold the finished chunk into the running sum (FP32, round to nearest): the
                 // accumulation error of the tensor core grows with the accumulated K, so no chunk
                 // accumulates more than 512 K16 steps
-                const int chunk = it / TC_CHUNK_STAGES;
+                const int chunk = it >> chunk_log2;
                 const bool waited = tc::mbar_wait(cdone, (chunk - 1) & 1, a.status);
                 // one decision per warp (tcgen05.ld / st are warp-collective); the warp's lanes stay
                 // together because every exit from this loop is decided per warp
@@ -444,7 +448,7 @@ __device__ __forceinline__ void tc_tile(const TcArgs& a, const int bx, const int
             const int TP = 2 * a.nr + 2;                // row pitch (floats): conflict-free columns
             const int quarter = warp & 3;
             const int row = quarter * 32 + lane, jr = row >> 1, ri = row & 1;
-            const bool chunked = nstages > TC_CHUNK_STAGES;  // earlier chunks are in the running sum
+            const bool chunked = nstages > chunk_mask + 1;  // earlier chunks are in the running sum
 #pragma unroll 1
             for (int ch = warp >> 2; ch * 32 < a.nr; ch += 4) {
                 float v[32];
@@ -495,10 +499,10 @@ __device__ __forceinline__ void tc_tile(const TcArgs& a, const int bx, const int
 }
 
 // grid (2 × pair tiles, readout tiles, voxel splits); CTAs 2i, 2i + 1 form a cluster
-template<bool JAC>
+template<bool JAC, bool SHORT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) tc_contract_kernel(TcArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    tc_tile<JAC>(a, blockIdx.x >> 1, blockIdx.y, blockIdx.z, smem_raw);
+    tc_tile<JAC, SHORT>(a, blockIdx.x >> 1, blockIdx.y, blockIdx.z, smem_raw);
 }
 
 // tile grid of one contraction: (pair tiles, readout tiles, voxel splits), 2 CTAs per tile
@@ -537,7 +541,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
         tile = make_int3(l2 % g.x, (l2 / g.x) % g.y, l2 / (g.x * g.y));
     }
     __syncthreads();
-    tc_tile<JAC>(job, tile.x, tile.y, tile.z, smem_raw);
+    tc_tile<JAC, true>(job, tile.x, tile.y, tile.z, smem_raw);
 }
 
 // batched tc_prep_kernel: flattened 128-thread block b → job j, voxel (b - offsets[j])·128 + t
@@ -601,6 +605,7 @@ int cartesian_tile(int nvoxels, int R, int S, int C, bool jac) {
 
 TcPlan tc_plan(int device, int nvoxels, int R, int S, int C, bool jac) {
     TcPlan p;
+    p.chunk_log2 = kernels::TC_CHUNK_LOG2;
     const TcTuning tuning = cartesian_tuning(nvoxels, R, S, C, jac);
     p.ntiles = div_ceil(C * S, kernels::TC_PAIRS);
     p.nr = cartesian_tile(nvoxels, R, S, C, jac);
@@ -620,32 +625,45 @@ TcPlan tc_plan(int device, int nvoxels, int R, int S, int C, bool jac) {
         // the partial tiles written and summed. It serves all products but small ones, which it leaves on a
         // few SMs (64 x 64 voxels, 400 readouts of one coil on 4 tiles: signal 24 us). The fine one: the least
         // estimated time of all counts, with what was measured on 117 shapes: 0.95 us a stage, 5.2 us a CTA (its
-        // pipeline's start and the drain), and the partials' sum, 3 us, 0.1 us a split and 0.32 us/MB (so that
-        // 1000 voxels, 200 readouts of 256 samples, 16 coils keep 2 splits: J·v 67 us, with 9 89 us). It
+        // pipeline's start and the drain), 0.7 us a fold, and the partials' sum, 3 us, 0.1 us a split and 0.32 us/MB (so that
+        // 1000 voxels, 200 readouts of 256 samples, 16 coils keep 2 splits: J·v 69 us, with 9 89 us). It
         // counts where the coarse grid is at most one CTA per SM and it estimates at least 5 % less.
+        // The accumulators are no longer (to the nearest power of two of stages) than splits of at least 4 stages that
+        // leave the least idle time would make them: fewer splits fold as often instead (that J·v: error against 64
+        // bits 4.6e-6, without the folds 8.2e-6, with 9 splits 4.6e-6).
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         const int stages = div_ceil(std::max(nvoxels, 1), vps);
         const double mb = 8e-6 * double(C) * S * R;
         auto waves = [&](int sp) { return double((int64_t(tiles) * sp + sms - 1) / sms); };
+        auto fullest = [&](int most) {
+            double best = -1.0;
+            int at = 1;
+            for (int sp = 1; sp <= std::max(1, std::min(64, most)); sp++) {
+                const double eff = double(int64_t(tiles) * sp) / (waves(sp) * sms) - 0.005 * sp;
+                if (eff > best + 1e-9) {
+                    best = eff;
+                    at = sp;
+                }
+            }
+            return at;
+        };
+        const int finest = div_ceil(stages, fullest(nvoxels / (4 * vps)));
+        int chunk_log2 = kernels::TC_CHUNK_LOG2;
+        while (chunk_log2 > 2 && 3 * finest < 2 * (1 << chunk_log2)) chunk_log2--;  // the nearest power of two
         auto estimate = [&](int sp) {
             const int per = div_ceil(stages, sp), n = div_ceil(stages, per);
-            return waves(n) * (0.95 * per + 5.2) + (n > 1 ? 3.0 + n * (0.1 + 0.32 * mb) : 0.0);
+            const int folds = per > finest ? (per - 1) >> chunk_log2 : 0;
+            return waves(n) * (0.95 * per + 5.2 + 0.7 * folds) + (n > 1 ? 3.0 + n * (0.1 + 0.32 * mb) : 0.0);
         };
-        double best = -1.0;
-        for (int sp = 1; sp <= std::max(1, std::min(64, nvoxels / (16 * vps))); sp++) {
-            const double eff = double(int64_t(tiles) * sp) / (waves(sp) * sms) - 0.005 * sp;
-            if (eff > best + 1e-9) {
-                best = eff;
-                splits = sp;
-            }
-        }
-        best = waves(splits) > 1.0 ? 0.0 : 0.95 * estimate(splits);
+        splits = fullest(nvoxels / (16 * vps));
+        double best = waves(splits) > 1.0 ? 0.0 : 0.95 * estimate(splits);
         for (int sp = 1; sp <= std::min(64, stages); sp++)
             if (estimate(sp) < best - 0.005) {
                 best = estimate(sp);
                 splits = sp;
             }
+        if (div_ceil(stages, splits) > finest) p.chunk_log2 = chunk_log2;
     }
     p.vchunk = std::max(vps, div_ceil(div_ceil(std::max(nvoxels, 1), splits), vps) * vps);
     p.splits = std::max(1, div_ceil(nvoxels, p.vchunk));
@@ -687,14 +705,26 @@ int tc_pack_blocks(int nr, int R, int apack_stages) {
 
 namespace {
 
+using TcKernel = void (*)(kernels::TcArgs);
+TcKernel tc_kernel(bool jac, int chunk_log2) {
+    if (chunk_log2 == kernels::TC_CHUNK_LOG2)
+        return jac ? kernels::tc_contract_kernel<true, false> : kernels::tc_contract_kernel<false, false>;
+    return jac ? kernels::tc_contract_kernel<true, true> : kernels::tc_contract_kernel<false, true>;
+}
+
 void set_tc_smem_attribute(bool jac, bool batch) {
     static std::once_flag once[4];
     std::call_once(once[int(jac) + 2 * int(batch)], [&] {
-        const void* fn = batch ? (jac ? reinterpret_cast<const void*>(kernels::tc_contract_batch_kernel<true>)
-                                      : reinterpret_cast<const void*>(kernels::tc_contract_batch_kernel<false>))
-                               : (jac ? reinterpret_cast<const void*>(kernels::tc_contract_kernel<true>)
-                                      : reinterpret_cast<const void*>(kernels::tc_contract_kernel<false>));
-        COMPAS_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kernels::TC_SMEM));
+        auto allow = [](const void* fn) {
+            COMPAS_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kernels::TC_SMEM));
+        };
+        if (batch) {
+            allow(jac ? reinterpret_cast<const void*>(kernels::tc_contract_batch_kernel<true>)
+                      : reinterpret_cast<const void*>(kernels::tc_contract_batch_kernel<false>));
+        } else {
+            allow(reinterpret_cast<const void*>(tc_kernel(jac, 0)));
+            allow(reinterpret_cast<const void*>(tc_kernel(jac, kernels::TC_CHUNK_LOG2)));
+        }
     });
 }
 
@@ -705,6 +735,7 @@ bool run_tc(const CompasContext& ctx, kernels::TcArgs a, bool jac, cfloat* out) 
     const TcPlan plan = tc_plan(ctx.device(), a.nvoxels, a.R, a.S, a.C, jac);
     const int splits = plan.splits;
     a.vchunk = plan.vchunk;
+    a.chunk_log2 = plan.chunk_log2;
     const int64_t n = int64_t(npairs) * a.R;
     Array<cfloat, 2> partials({splits > 1 ? splits : 0, n}, ctx.device(), ctx.stream());
     const TcTables tables = tc_tables(a.nvoxels, a.R, a.S, a.C, jac);
@@ -722,7 +753,7 @@ bool run_tc(const CompasContext& ctx, kernels::TcArgs a, bool jac, cfloat* out) 
         kernels::tc_pack_a_kernel<false><<<pgrid, 256, 0, ctx.stream()>>>(a);
     }
     check_launch("tc_prep_kernel / tc_pack_a_kernel");
-    auto fn = jac ? kernels::tc_contract_kernel<true> : kernels::tc_contract_kernel<false>;
+    const TcKernel fn = tc_kernel(jac, a.chunk_log2);
     set_tc_smem_attribute(jac, false);
     dim3 grid(2 * plan.ntiles, plan.mtiles, splits);
     fn<<<grid, kernels::TC_THREADS, kernels::TC_SMEM, ctx.stream()>>>(a);
