@@ -37,22 +37,29 @@ std::mutex g_mutex;
 DeviceState g_devices[kMaxDevices];
 
 // The words of detail::HostFlag: one block for the process, made with the first context and kept to its end
-// (a kernel may still write to a word whose flag is gone). A sequence beyond their number runs
-// without one: its calls launch both forms.
+// (a kernel may still write to a word whose flag is gone, and a flag may outlive the library's statics). A sequence
+// beyond their number runs without one: its calls launch both forms.
 constexpr int kHostFlags = 1024;
-std::mutex g_flag_mutex;
-unsigned int* g_flag_words = nullptr;
-std::vector<unsigned int*> g_flag_free;
-unsigned int g_flag_ticket = 0;
+struct HostFlags {
+    std::mutex mutex;
+    unsigned int* words = nullptr;
+    std::vector<unsigned int*> free;
+    unsigned int ticket = 0;
+};
+HostFlags& host_flags() {
+    static HostFlags* flags = new HostFlags;
+    return *flags;
+}
 
 void make_host_flags() {
-    std::lock_guard<std::mutex> lock(g_flag_mutex);
-    if (g_flag_words != nullptr) return;
+    HostFlags& f = host_flags();
+    std::lock_guard<std::mutex> lock(f.mutex);
+    if (f.words != nullptr) return;
     void* p = nullptr;
     COMPAS_CUDA_CHECK(cudaHostAlloc(&p, kHostFlags * sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped));
-    g_flag_words = static_cast<unsigned int*>(p);
-    g_flag_free.reserve(kHostFlags);
-    for (int i = kHostFlags - 1; i >= 0; i--) g_flag_free.push_back(g_flag_words + i);
+    f.words = static_cast<unsigned int*>(p);
+    f.free.reserve(kHostFlags);
+    for (int i = kHostFlags - 1; i >= 0; i--) f.free.push_back(f.words + i);
 }
 
 DeviceState& device_state(int device) {
@@ -108,22 +115,24 @@ unsigned int* device_status_word(int device) {
 }
 
 HostFlag::HostFlag() : m_word(nullptr), m_ticket(0) {
-    std::lock_guard<std::mutex> lock(g_flag_mutex);
-    if (g_flag_free.empty()) return;
-    m_word = g_flag_free.back();
-    g_flag_free.pop_back();
+    HostFlags& f = host_flags();
+    std::lock_guard<std::mutex> lock(f.mutex);
+    if (f.free.empty()) return;
+    m_word = f.free.back();
+    f.free.pop_back();
     // 31 bits, never 0: what a word holds from its earlier users, or gets from their kernels still, is
     // another ticket's and reads as unknown
-    g_flag_ticket = (g_flag_ticket + 1) & 0x7fffffffu;
-    if (g_flag_ticket == 0) g_flag_ticket = 1;
-    m_ticket = g_flag_ticket;
+    f.ticket = (f.ticket + 1) & 0x7fffffffu;
+    if (f.ticket == 0) f.ticket = 1;
+    m_ticket = f.ticket;
     *static_cast<volatile unsigned int*>(m_word) = 0;
 }
 
 HostFlag::~HostFlag() {
     if (m_word == nullptr) return;
-    std::lock_guard<std::mutex> lock(g_flag_mutex);
-    g_flag_free.push_back(m_word);
+    HostFlags& f = host_flags();
+    std::lock_guard<std::mutex> lock(f.mutex);
+    f.free.push_back(m_word);
 }
 
 int HostFlag::value() const {
