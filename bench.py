@@ -62,14 +62,17 @@ def load_peaks():
         return FALLBACK_PEAKS, "fallback"
 
 
-def profile_traffic(name):
+def profile_traffic(name, voxels=None):
     """DRAM bytes per launch from a committed ncu summary (profiles/<name>.txt, line
-    'dram_bytes_per_launch: <n>'), or None."""
+    'dram_bytes_per_launch: <n> (<voxels> voxels)'), or None; also None when the capture was of another
+    number of voxels than `voxels`."""
     p = ROOT / "profiles" / f"{name}.txt"
     if not p.exists():
         return None
     for line in p.read_text().splitlines():
         if line.startswith("dram_bytes_per_launch:"):
+            if voxels is not None and f"({voxels} voxels)" not in line:
+                return None
             try:
                 return float(line.split(":", 1)[1].split()[0])
             except ValueError:
@@ -392,7 +395,7 @@ def main():
     exec_frac = lane_ops / (sim_ms / 1e3) / (148 * 128 * f_mhz * 1e6)
     roofline = {"bound": "fp32", "kernel": "fisp_real_kernel" if real_phases else "fisp_epg_kernel", "achieved": epg_tf, "peak": fp32_peak_tf,
                 "unit": "TFLOP/s", "frac": epg_tf / fp32_peak_tf,
-                "traffic": profile_traffic("fisp_real_mrstat" if real_phases else "fisp_epg_mrstat"),
+                "traffic": profile_traffic("fisp_real_mrstat", Vl) if real_phases else None,
                 "executed": {"fp32_lane_ops_per_voxel_position_tr": per_item, "layout": layout,
                              "real_phase_form": real_phases,
                              "fp32_lane_ops": lane_ops, "frac_of_fp32_peak": exec_frac},

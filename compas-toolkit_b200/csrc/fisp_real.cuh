@@ -20,9 +20,9 @@
 // spoiling, which stays on the general kernels (fisp_real_covers).
 //
 // Bound by the FP32 pipe (182 lane operations per voxel, position and TR at 25 states: 12 pairs of 14, state 0
-// and the coefficients). MR-STAT slice (50176 voxels, 1120 TRs, 25 states, 35 positions): 12.7 ms,
+// and the coefficients). MR-STAT slice (50176 voxels, 1120 TRs, 25 states, 35 positions): 12.6 ms,
 // 41.7 ms as complex states; its tangents at 9216 voxels: 9.9 ms, 42.7 ms before; 4096 voxels, 400 TRs,
-// 8 states, 1 position: 38 us, 113 us before. The two-wide instructions of the states run at 86 % of the
+// 8 states, 1 position: 35 us, 113 us before. The two-wide instructions of the states run at 86 % of the
 // pipe's rate (8 against 25 states; ncu: pipe 76 % busy overall); the scalar forms of the same operations,
 // all or every second pair, ran 5-10 % slower.
 #pragma once

@@ -19,11 +19,11 @@
 // cheapest of three loops that does what all its voxels need; in each of them a voxel gets the same bits
 // (what it does not need enters as a factor of 1 or a highest coefficient of 0), so its echoes
 // do not depend on its neighbours. Loop 2, in us for 20000 voxels, 60 TRs of 15 samples, 9 / 35 z (with the
-// 24-operation rotation in brackets): 30 % of the voxels with T2 = 0 338 / 662 (350 / 729; no such voxel, loop
-// 0: 170 / 394), az of 1 rad at the outer z 549 / 1523 (1349 / 2810); pulses of one sample of 40° 61 / 125 (139 / 219).
+// 24-operation rotation in brackets): 30 % of the voxels with T2 = 0 293 / 588 (350 / 729; no such voxel, loop
+// 0: 166 / 388), az of 1 rad at the outer z 488 / 1077 (1349 / 2810); pulses of one sample of 40° 53 / 115 (139 / 219).
 //
 // Bound by the FP32 pipe. 35 z, 15 RF samples: 50176 voxels, 320 TRs 4.85 ms (7.93 ms with the 24-operation
-// rotation), tangents at 100 TRs 4.0 ms (6.3); 2500 voxels, 743 TRs 1.35 ms (3.37). The loop over the samples
+// rotation), tangents at 100 TRs 3.25 ms (6.3); 2500 voxels, 743 TRs 1.34 ms (3.37). The loop over the samples
 // holds an even and an odd body and a third for the last sample of an odd count: with a branch in
 // the loop instead, 10 % slower.
 #pragma once
