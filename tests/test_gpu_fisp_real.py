@@ -217,3 +217,17 @@ def test_more_sequences_than_flags_and_reused_flags(cb, ctx):
             for i, g in enumerate(got):
                 assert np.array_equal(g.to_numpy(), ref[(i + shift) % 2]), i
         del kept, got
+
+
+@pytest.mark.parametrize("kind", ["fisp", "pssfp"])
+@pytest.mark.parametrize("turned", [False, True])
+def test_threads_that_share_a_new_sequence(cb, ctx, kind, turned):
+    # the first calls, which do not know the form yet, and later ones from four threads at once
+    from concurrent.futures import ThreadPoolExecutor
+
+    params = cb.TissueParameters.from_soa(ctx, W.tissue_voxels(np.random.default_rng(2), 70, 22.4))
+    ref = cb.simulate_magnetization(ctx, params, _sequence(cb, ctx, kind, turned)).to_numpy()
+    s = _sequence(cb, ctx, kind, turned)
+    with ThreadPoolExecutor(4) as pool:
+        for got in pool.map(lambda _: cb.simulate_magnetization(ctx, params, s).to_numpy(), range(200)):
+            assert np.array_equal(got, ref)
